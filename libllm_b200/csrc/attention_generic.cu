@@ -3,9 +3,16 @@
 // optional block mask (a query sees only keys of its own block of `block` positions, blocks
 // counted from position 0), optionally the first `sink` positions of the sequence kept visible
 // beyond the window (at their true positions), optional gate per (token, head) on the result (multiplied by
-// sigmoid(gate)); element type float or bfloat16, arithmetic in 32-bit.  One warp serves one (token, head): lanes take 32 keys at a time
-// for the scores, then 32 channels at a time for the weighted sum, with a running
-// maximum and sum (the online form of softmax, src/flint/cpu/softmax.cc:31-60).
+// sigmoid(gate)); element type float or bfloat16, arithmetic in 32-bit.  A CTA of four warps serves one (token, head): the
+// warps take blocks of 32 keys in turn, lanes a key each for the scores, then 32 channels at a time for the
+// weighted sum, with a running maximum and sum per warp (the online form of softmax,
+// src/flint/cpu/softmax.cc:31-60); the four are joined in warp order.
+//
+// What bounds it is a warp's chain of loads, a few hundred keys long in a decoding step whose 64 or so (token, head) pairs
+// leave most SMs without a warp: hence four warps to a pair, eight value rows asked for before the first is
+// used, a key's place in the pages worked out once by the lane that scores it, and loops over
+// channels no longer than the head (instantiations for heads up to 64, 128, 256 and 1,024).
+// 32 heads of 64 over 8 key heads, two sequences of some 150 keys: 158 -> 17 us a launch (prompt and single tokens together).
 //
 // This is the attention of the true 32-bit path and of head sizes the fast bfloat16
 // kernels do not take.  It serves prompts and single tokens alike: the keys of the
@@ -23,7 +30,7 @@
 LLM_DEFINE_LAST_ERROR(llm_attention_generic_last_error)
 
 constexpr int WARPS = 4;
-constexpr int MAX_D_SMALL = 256, MAX_D_LARGE = 1024;
+constexpr int MAX_D_LARGE = 1024;
 
 __device__ __forceinline__ float dot_row(const float *q, const float *k, int d, bool vec) {
   float acc = 0.f;
@@ -31,6 +38,7 @@ __device__ __forceinline__ float dot_row(const float *q, const float *k, int d, 
     for (int c = 0; c < d; ++c) acc = fmaf(q[c], k[c], acc);
     return acc;
   }
+#pragma unroll 4
   for (int c = 0; c < d; c += 4) {
     const float4 v = *reinterpret_cast<const float4 *>(k + c);
     acc = fmaf(q[c], v.x, acc);
@@ -46,6 +54,7 @@ __device__ __forceinline__ float dot_row(const float *q, const __nv_bfloat16 *k,
     for (int c = 0; c < d; ++c) acc = fmaf(q[c], __bfloat162float(k[c]), acc);
     return acc;
   }
+#pragma unroll 2
   for (int c = 0; c < d; c += 8) {
     const uint4 raw = *reinterpret_cast<const uint4 *>(k + c);
     const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw);
@@ -72,43 +81,43 @@ attention_generic_kernel(const T *__restrict__ q, long long q_stride, T *__restr
                          long long out_stride, const T *__restrict__ kcache,
                          const T *__restrict__ vcache, const int *__restrict__ tok_seq,
                          const int *__restrict__ tok_pos, const int *__restrict__ page_table,
-                         int pt_stride, int n_tokens, int n_heads, int n_kv, int d, int dv, int page_size,
+                         int pt_stride, int n_heads, int n_kv, int d, int dv, int page_size,
                          int window, int block, int sink, float scale, const float *__restrict__ gate,
                          long long gate_stride, int vec, int v_ld, float null_score, const float *__restrict__ null_scores,
                          SigmoidWeights sig) {
-  __shared__ __align__(16) float q_s[WARPS][MAX_D];
+  __shared__ __align__(16) float q_s[MAX_D];
+  __shared__ float acc_s[WARPS][MAX_D];
+  __shared__ float m_s[WARPS], l_s[WARPS];
+  constexpr int NI = MAX_D / 32, AHEAD = MAX_D <= 256 ? 8 : 2;     // value rows on their way at once
+  grid_dependents_launch();
+  grid_dependency_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long w = (long long)blockIdx.x * WARPS + warp;
-  const int token = (int)(w / n_heads), h = (int)(w % n_heads);
-  if (token >= n_tokens) return;
+  const int token = (int)(blockIdx.x / (unsigned)n_heads), h = (int)(blockIdx.x % (unsigned)n_heads);
   const int p = tok_pos[token];
   const int *pt = page_table + (size_t)tok_seq[token] * pt_stride;
   const int kvh = h / (n_heads / n_kv);
   const T *qrow = q + (size_t)token * q_stride + (size_t)h * d;
-  for (int c = lane; c < d; c += 32) q_s[warp][c] = to_float(qrow[c]);
-  __syncwarp();
+  for (int c = threadIdx.x; c < d; c += WARPS * 32) q_s[c] = to_float(qrow[c]);
+  __syncthreads();
 
   int kstart = window > 0 ? max(0, p - window + 1) : 0;
   if (block > 0) kstart = max(kstart, p / block * block);
   float m = -INFINITY, l = 0.f;
   const float temp = SIG ? sig.temp[h] : 0.f, bias = SIG ? sig.bias[h] : 0.f;
-  float acc[MAX_D / 32];
+  float acc[NI];
 #pragma unroll
-  for (int i = 0; i < MAX_D / 32; ++i) acc[i] = 0.f;
+  for (int i = 0; i < NI; ++i) acc[i] = 0.f;
 
   // two runs of keys: the kept first positions that lie before the window, then the window
   const int sink_end = (window > 0 && block == 0) ? min(sink, kstart) : 0;
   for (int run = sink_end > 0 ? 0 : 1; run < 2; ++run) {
     const int k0 = run == 0 ? 0 : kstart, k1 = run == 0 ? sink_end : p + 1;
-    for (int kb = k0; kb < k1; kb += 32) {
-      const int j = kb + lane;
-      const bool valid = j < k1;
+    for (int kb = k0 + warp * 32; kb < k1; kb += WARPS * 32) {
+      const int j = min(kb + lane, k1 - 1);
+      const bool valid = kb + lane < k1;
+      const long long at = ((long long)pt[j / page_size] * n_kv + kvh) * page_size + j % page_size;   // this lane's key's row
       float s = -INFINITY;
-      if (valid) {
-        const int page = pt[j / page_size];
-        const T *krow = kcache + (((size_t)page * n_kv + kvh) * page_size + (j % page_size)) * d;
-        s = dot_row(q_s[warp], krow, d, vec != 0) * scale;
-      }
+      if (valid) s = dot_row(q_s, kcache + at * d, d, vec != 0) * scale;
       float pj;
       if (SIG) {
         s *= temp;
@@ -120,37 +129,57 @@ attention_generic_kernel(const T *__restrict__ q, long long q_stride, T *__restr
         const float alpha = expf(m - m_new);                // 0 on the first block (m = -inf)
         l = l * alpha + warp_sum(pj);
 #pragma unroll
-        for (int i = 0; i < MAX_D / 32; ++i) acc[i] *= alpha;
+        for (int i = 0; i < NI; ++i) acc[i] *= alpha;
         m = m_new;
       }
       const int nvalid = min(32, k1 - kb);
-      for (int jj = 0; jj < nvalid; ++jj) {
-        const float pv = __shfl_sync(0xffffffffu, pj, jj);
-        const int key = kb + jj;
-        const int page = pt[key / page_size];
-        const T *vrow = vcache + (((size_t)page * n_kv + kvh) * page_size + (key % page_size)) * v_ld;
+      for (int j0 = 0; j0 < nvalid; j0 += AHEAD) {
+        float v[AHEAD][NI];
 #pragma unroll
-        for (int i = 0; i < MAX_D / 32; ++i) {
-          const int c = lane + 32 * i;
-          if (c < dv) acc[i] = fmaf(pv, to_float(vrow[c]), acc[i]);
+        for (int u = 0; u < AHEAD; ++u) {
+          const T *vrow = vcache + __shfl_sync(0xffffffffu, at, j0 + u) * v_ld;       // beyond nvalid: the last key's row, not used
+#pragma unroll
+          for (int i = 0; i < NI; ++i) v[u][i] = lane + 32 * i < dv ? to_float(vrow[lane + 32 * i]) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+          const float pv = __shfl_sync(0xffffffffu, pj, j0 + u);
+          if (j0 + u < nvalid) {
+#pragma unroll
+            for (int i = 0; i < NI; ++i) acc[i] = fmaf(pv, v[u][i], acc[i]);
+          }
         }
       }
     }
   }
-  T *orow = out + (size_t)token * out_stride + (size_t)h * dv;
-  if (null_scores) null_score = null_scores[h];
-  if (!SIG && null_score > -INFINITY) {     // one more key whose score is null_score and whose value is nought
-    const float m_new = fmaxf(m, null_score), alpha = expf(m - m_new);
-    l = l * alpha + expf(null_score - m_new);
 #pragma unroll
-    for (int i = 0; i < MAX_D / 32; ++i) acc[i] *= alpha;
+  for (int i = 0; i < NI; ++i) acc_s[warp][lane + 32 * i] = acc[i];
+  if (lane == 0) {
+    m_s[warp] = m;
+    l_s[warp] = l;
   }
-  float inv = SIG ? sig.out_scale : 1.f / l;
-  if (gate) inv *= 1.f / (1.f + expf(-gate[(size_t)token * gate_stride + h]));
+  __syncthreads();
+  if (null_scores) null_score = null_scores[h];
+  float top = -INFINITY;
+  if (!SIG) {
 #pragma unroll
-  for (int i = 0; i < MAX_D / 32; ++i) {
-    const int c = lane + 32 * i;
-    if (c < dv) orow[c] = from_float<T>(acc[i] * inv);
+    for (int w = 0; w < WARPS; ++w) top = fmaxf(top, m_s[w]);
+    top = fmaxf(top, null_score);           // one more key whose score is null_score and whose value is nought, if above -inf
+  }
+  float f[WARPS], sum = !SIG && null_score > -INFINITY ? expf(null_score - top) : 0.f;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    f[w] = SIG ? 1.f : m_s[w] == -INFINITY ? 0.f : expf(m_s[w] - top);
+    sum += l_s[w] * f[w];
+  }
+  float inv = SIG ? sig.out_scale : 1.f / sum;
+  if (gate) inv *= 1.f / (1.f + expf(-gate[(size_t)token * gate_stride + h]));
+  T *orow = out + (size_t)token * out_stride + (size_t)h * dv;
+  for (int c = threadIdx.x; c < dv; c += WARPS * 32) {
+    float o = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) o = fmaf(acc_s[w][c], f[w], o);
+    orow[c] = from_float<T>(o * inv);
   }
 }
 
@@ -172,27 +201,35 @@ static int launch_generic(int dtype, const void *q, long long q_stride, void *ou
   LLM_REQUIRE(sink == 0 || block == 0, "attention: kept first positions go with a window, not with a block mask");
   // 16-byte loads of key rows where rows start on such a boundary
   const int vec = (dtype == LLM_F32 ? d % 4 == 0 : d % 8 == 0) && (uintptr_t)kcache % 16 == 0;
-  const long long warps = (long long)n_tokens * n_heads;
-  const long long blocks = (warps + WARPS - 1) / WARPS;
+  const long long blocks = (long long)n_tokens * n_heads;
   LLM_REQUIRE(blocks < 2147483647LL, "attention: too many tokens for one launch");
-  const bool small = d <= MAX_D_SMALL && dv <= MAX_D_SMALL;
+  const int widest = d > dv ? d : dv;
   const SigmoidWeights sw = sig ? *sig : SigmoidWeights{};
-#define GENERIC_GO(T, MAXD)                                                                                              \
-  if (sig) GENERIC_RUN(T, MAXD, true);                                                                                   \
-  else GENERIC_RUN(T, MAXD, false)
 #define GENERIC_RUN(T, MAXD, SIG)                                                                                        \
-  attention_generic_kernel<T, MAXD, SIG><<<(unsigned)blocks, WARPS * 32, 0, stream>>>(                                          \
-      (const T *)q, q_stride, (T *)out, out_stride, (const T *)kcache, (const T *)vcache, tok_seq, tok_pos, page_table, pt_stride, \
-      n_tokens, n_heads, n_kv, d, dv, page_size, window, block, sink, scale, gate, gate_stride, vec, v_ld, null_score, null_scores, sw)
-  if (dtype == LLM_F32 && small) { GENERIC_GO(float, MAX_D_SMALL); }
-  else if (dtype == LLM_F32) { GENERIC_GO(float, MAX_D_LARGE); }
-  else if (dtype == LLM_BF16 && small) { GENERIC_GO(__nv_bfloat16, MAX_D_SMALL); }
-  else if (dtype == LLM_BF16) { GENERIC_GO(__nv_bfloat16, MAX_D_LARGE); }
-  else LLM_FAIL("attention: unknown dtype %d", dtype);
-#undef GENERIC_RUN
+  LLM_CHECK_CUDA(llm_launch(attention_generic_kernel<T, MAXD, SIG>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,      \
+                            (const T *)q, q_stride, (T *)out, out_stride, (const T *)kcache, (const T *)vcache, tok_seq, tok_pos, page_table,  \
+                            pt_stride, n_heads, n_kv, d, dv, page_size, window, block, sink, scale, gate, gate_stride, vec, v_ld,     \
+                            null_score, null_scores, sw),                                                                \
+                 "attention_generic")
+#define GENERIC_GO(T, MAXD)                                                                                              \
+  do {                                                                                                                   \
+    if (sig) GENERIC_RUN(T, MAXD, true);                                                                                 \
+    else GENERIC_RUN(T, MAXD, false);                                                                                    \
+    return LLM_OK;                                                                                                       \
+  } while (0)
+#define GENERIC_TYPE(T)                                                                                                  \
+  do {                                                                                                                   \
+    if (widest <= 64) GENERIC_GO(T, 64);                                                                                 \
+    if (widest <= 128) GENERIC_GO(T, 128);                                                                               \
+    if (widest <= 256) GENERIC_GO(T, 256);                                                                               \
+    GENERIC_GO(T, MAX_D_LARGE);                                                                                          \
+  } while (0)
+  if (dtype == LLM_F32) GENERIC_TYPE(float);
+  if (dtype == LLM_BF16) GENERIC_TYPE(__nv_bfloat16);
+  LLM_FAIL("attention: unknown dtype %d", dtype);
+#undef GENERIC_TYPE
 #undef GENERIC_GO
-  LLM_CHECK_LAUNCH("attention_generic");
-  return LLM_OK;
+#undef GENERIC_RUN
 }
 
 LLM_EXPORT int llm_attention_generic_ld(int dtype, const void *q, long long q_stride, void *out,

@@ -470,6 +470,27 @@ def test_tensor_core_product_in_parts_of_k(M, N, K, parts):
     assert 1 <= ops.gemm_tc_suggest_parts(M, N, K) <= 8
 
 
+# one part with work and eight, parts that end inside a block, widths beside the tiles; 4-byte rows take the general kernel
+@pytest.mark.parametrize("K,N", [(4, 1), (36, 15), (252, 16), (260, 17), (1028, 130), (2048, 64), (97, 33)])
+def test_32_bit_product_rows_do_not_depend_on_the_batch(K, N):
+    """Every number of rows at which another kernel takes over gives a row the same bits, and rounding alone lies between
+    them and 64 bits: each part adds at most K / 8 + 32 products one behind the other."""
+    from libllm_b200.csrc import ops
+    a = rnd((130, K), "float32", 91)
+    w = rnd((N, K), "float32", 92)
+    bias = rnd((N,), "float32", 93)
+    rows = {}
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 130):
+        out = torch.full((M, N), float("nan"), dtype=torch.float32, device=DEV)
+        ops.gemm_plain(a[:M], w, out, bias)
+        rows[M] = out
+    ref = a.double() @ w.double().T + bias.double()
+    bound = (K / 8 + 40) * 2 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double()) if K % 4 == 0 else K * 2 ** -24 * (a.abs().double() @ w.abs().double().T + 1)
+    assert bool(((rows[130].double() - ref).abs() <= bound).all())
+    for M, out in rows.items():
+        assert torch.equal(out, rows[130][:M]), M
+
+
 @pytest.mark.parametrize("M,I,K", [(1, 64, 64), (5, 173, 80), (8, 8192, 2048), (40, 300, 256), (200, 128, 136), (257, 391, 200),
                                    (1000, 1024, 512)])
 def test_tensor_core_product_with_swiglu(M, I, K):
