@@ -411,21 +411,29 @@ latent_decode_kernel(const __nv_bfloat16 *__restrict__ qa, long long ldq, const 
     return;
   }
 
+  // A warp fetches whole rows, so that a row's place in the pages is worked out once and not by each of its 16-byte pieces: what
+  // the loads cost was the divisions and page lookups around each of them.
   auto load_rows = [&](int kt, int stage) {
     __nv_bfloat16 *tk = sK + stage * LT_BN * ldr;
-    for (int c = tid; c < LT_BN * rch; c += LD_WARPS * 32) {
-      const int r = c / rch, ch = c - r * rch;
+#pragma unroll 4
+    for (int r = warp; r < LT_BN; r += LD_WARPS) {
       const int j = kt * LT_BN + r;
-      const bool ok = j >= kstart && j < len && ch < row8;
-      const int jj = j >= kstart && j < len ? j : pos;       // a page before the window may have been given back
-      const __nv_bfloat16 *src = cache + ((size_t)pt[jj / page_size] * page_size + jj % page_size) * (size_t)row + (ok ? ch : 0) * 8;
-      cp_async16(tk + r * ldr + ch * 8, src, ok);
+      const bool seen = j >= kstart && j < len;
+      const int jj = seen ? j : pos;                         // a page before the window may have been given back
+      const __nv_bfloat16 *src = cache + ((size_t)pt[jj / page_size] * page_size + jj % page_size) * (size_t)row;
+      for (int ch = lane; ch < rch; ch += 32) {
+        const bool ok = seen && ch < row8;
+        cp_async16(tk + r * ldr + ch * 8, src + (ok ? ch : 0) * 8, ok);
+      }
     }
   };
-  for (int c = tid; c < LD_HT * rch; c += LD_WARPS * 32) {
-    const int r = c / rch, ch = c - r * rch;
-    const bool ok = h0 + r < n_heads && ch < row8;
-    cp_async16(sQ + r * ldr + ch * 8, ok ? qa + (size_t)tok * ldq + (size_t)(h0 + r) * row + ch * 8 : qa, ok);
+#pragma unroll 4
+  for (int r = warp; r < LD_HT; r += LD_WARPS) {
+    const __nv_bfloat16 *src = h0 + r < n_heads ? qa + (size_t)tok * ldq + (size_t)(h0 + r) * row : qa;
+    for (int ch = lane; ch < rch; ch += 32) {
+      const bool ok = h0 + r < n_heads && ch < row8;
+      cp_async16(sQ + r * ldr + ch * 8, src + (ok ? ch : 0) * 8, ok);
+    }
   }
   load_rows(kt0, 0);
   cp_async_commit();

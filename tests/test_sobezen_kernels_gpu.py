@@ -206,3 +206,48 @@ def test_latent_prompt_and_token_by_token_are_one_function(sizes):
     for other in results[1:]:
         for i in range(2):
             close(other[i][0], results[0][i][0].double(), "bfloat16", f"latent layer {i} in single tokens", roundings=4.0)
+
+
+# tokens at which another instantiation takes over, heads of one and of several fetches of w_uk, latents with an odd width
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T,H,d,rot,R,dv", [(1, 2, 6, 2, 22, 10), (2, 3, 64, 32, 512, 64), (3, 1, 65, 0, 33, 7), (4, 2, 80, 4, 520, 9),
+                                            (5, 2, 64, 8, 130, 64), (9, 1, 130, 6, 48, 24), (17, 2, 33, 2, 600, 5)])
+def test_queries_take_in_the_keys_matrix_and_results_are_expanded(T, H, d, rot, R, dv, dtype):
+    """latent_absorb and latent_expand against 64 bits: a sum of n products is off by at most n + 2 roundings of its terms'
+    absolute sum, and a 16-bit result by one of its own."""
+    from ctypes import c_int, c_longlong, c_void_p
+    from libllm_b200.csrc import ops
+    g = torch.Generator().manual_seed(T * R + d)
+    row, dt = R + rot, DT[dtype]
+    q = torch.randn(T, H * (d + rot), generator=g)
+    w_uk, w_uv = (torch.randn(H * n, R, generator=g).to(dt) for n in (d, dv))
+    table = torch.randn(9, max(rot, 1), generator=g)
+    pos = torch.randint(0, 9, (T,), generator=g).int()
+    out = torch.full((T, H * row), float("nan"), dtype=dt, device=DEV)
+    dev = [t.to(DEV) for t in (q, w_uk, table, pos, w_uv)]
+    stream = torch.cuda.current_stream().cuda_stream
+    code = 0 if dtype == "float32" else 1
+    ops._call("latent", "llm_latent_absorb",
+              [c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong] + [c_int] * 5 + [c_void_p, c_int, c_int, c_void_p, c_void_p],
+              code, dev[0].data_ptr(), q.shape[1], dev[1].data_ptr(), out.data_ptr(), H * row, T, H, d, rot, R, dev[2].data_ptr(), 9, 1,
+              dev[3].data_ptr(), stream)
+    got, q3 = out.cpu().double().view(T, H, row), q.double().view(T, H, d + rot)
+    w3 = w_uk.double().view(H, d, R)
+    result = 2 ** -8 if dtype == "bfloat16" else 0.0
+    ref = torch.einsum("thi,hic->thc", q3[..., :d], w3)
+    room = (d + 2) * 2 ** -24 * torch.einsum("thi,hic->thc", q3[..., :d].abs(), w3.abs()) + result * ref.abs()
+    assert bool(((got[..., :R] - ref).abs() <= room).all())
+    if rot:
+        a, b = q3[..., d::2], q3[..., d + 1::2]
+        c, s = (table[pos.long()].double()[:, None, i * rot // 2:(i + 1) * rot // 2] for i in range(2))
+        for part_, want in ((got[..., R::2], a * c - b * s), (got[..., R + 1::2], b * c + a * s)):
+            assert bool(((part_ - want).abs() <= 4 * 2 ** -24 * (a.abs() * c.abs().maximum(s.abs()) + b.abs() * c.abs().maximum(s.abs())) + result * want.abs()).all())
+    x = torch.randn(T, H * R, generator=g).to(dt)
+    y = torch.full((T, H * dv), float("nan"), dtype=dt, device=DEV)
+    xd = x.to(DEV)
+    ops._call("latent", "llm_latent_expand", [c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong] + [c_int] * 4 + [c_void_p],
+              code, xd.data_ptr(), H * R, dev[4].data_ptr(), y.data_ptr(), H * dv, T, H, R, dv, stream)
+    x3, v3 = x.double().view(T, H, R), w_uv.double().view(H, dv, R)
+    ref = torch.einsum("thc,hjc->thj", x3, v3)
+    room = (R / 32 + 8) * 2 ** -24 * torch.einsum("thc,hjc->thj", x3.abs(), v3.abs()) + result * ref.abs()
+    assert bool(((y.cpu().double().view(T, H, dv) - ref).abs() <= room).all())
