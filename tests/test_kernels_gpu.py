@@ -470,6 +470,31 @@ def test_tensor_core_product_in_parts_of_k(M, N, K, parts):
     assert 1 <= ops.gemm_tc_suggest_parts(M, N, K) <= 8
 
 
+# widths at and beside a lane's pieces, the row count at which the prompt kernel takes over and one that leaves a CTA's last warps idle
+@pytest.mark.parametrize("hidden", [516, 1024, 1028, 2048, 2052, 3072, 4092, 4096])
+@pytest.mark.parametrize("parts,scaled", [(0, False), (1, False), (1, True)])
+def test_norm_of_prompt_rows_has_the_bits_of_a_row_alone(hidden, parts, scaled):
+    from ctypes import c_float, c_int, c_longlong, c_void_p
+    from libllm_b200.csrc import ops
+    rows = 1027
+    x, w = rnd((rows, hidden), "float32", 94), rnd((hidden,), "float32", 95)
+    delta = rnd((rows, hidden), "float32", 96) if parts else None
+    cs, cb = (rnd((hidden,), "float32", 97), rnd((hidden,), "float32", 98)) if scaled else (None, None)
+    got, one = torch.empty((rows, hidden), dtype=torch.bfloat16, device=DEV), torch.empty((3, hidden), dtype=torch.bfloat16, device=DEV)
+    a, b = x.clone(), x[[0, 517, 1026]].contiguous()
+    P_, I_ = c_void_p, c_int
+    call = lambda r, d, o: ops._call(  # noqa: E731
+        "elementwise", "llm_add_rmsnorm_scaled", [P_, P_, I_, I_, c_longlong, P_, c_float, P_, I_, P_, I_, I_, P_, P_, P_],
+        r.data_ptr(), d.data_ptr() if d is not None else None, 0, parts, r.numel(), w.data_ptr(), 1e-5, o.data_ptr(), 1, None, r.shape[0], hidden,
+        cs.data_ptr() if scaled else None, cb.data_ptr() if scaled else None, torch.cuda.current_stream().cuda_stream)
+    call(a, delta, got)
+    call(b, delta[[0, 517, 1026]].contiguous() if parts else None, one)
+    assert torch.equal(a[[0, 517, 1026]], b) and torch.equal(got[[0, 517, 1026]], one)
+    v = x.double() + (0 if not parts else (delta.double() + cb.double()) * cs.double() if scaled else delta.double())
+    ref = v / (v * v).mean(-1, keepdim=True).add(1e-5).sqrt() * w.double()
+    assert bool(((got.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all())
+
+
 # one part with work and eight, parts that end inside a block, widths beside the tiles; 4-byte rows take the general kernel
 @pytest.mark.parametrize("K,N", [(4, 1), (36, 15), (252, 16), (260, 17), (1028, 130), (2048, 64), (97, 33)])
 def test_32_bit_product_rows_do_not_depend_on_the_batch(K, N):
