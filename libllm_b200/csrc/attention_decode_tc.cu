@@ -381,6 +381,7 @@ attention_decode_tc_kernel(const float *__restrict__ qkv, long long qkv_stride, 
   float *sm_o = reinterpret_cast<float *>(sK);                 // [4][16][DV], over the tiles (no longer read)
   {
     const int ra = g, rb = g + 8;
+    // rows beyond the group are zeros nobody reads
     if (t == 0) {
       sm_m[warp][ra] = m_run[0] == -INFINITY ? -INFINITY : m_run[0] * scale_log2;
       sm_m[warp][rb] = m_run[1] == -INFINITY ? -INFINITY : m_run[1] * scale_log2;
@@ -391,10 +392,8 @@ attention_decode_tc_kernel(const float *__restrict__ qkv, long long qkv_stride, 
     for (int i = 0; i < DT; ++i) {
       float *pa = sm_o + ((size_t)(warp * DT_ROWS + ra) * DV + i * 8 + 2 * t);
       float *pb = sm_o + ((size_t)(warp * DT_ROWS + rb) * DV + i * 8 + 2 * t);
-      pa[0] = o[i][0];
-      pa[1] = o[i][1];
-      pb[0] = o[i][2];
-      pb[1] = o[i][3];
+      if (ra < G) *reinterpret_cast<float2 *>(pa) = make_float2(o[i][0], o[i][1]);
+      if (rb < G) *reinterpret_cast<float2 *>(pb) = make_float2(o[i][2], o[i][3]);
     }
   }
   __syncthreads();
@@ -427,17 +426,20 @@ attention_decode_tc_kernel(const float *__restrict__ qkv, long long qkv_stride, 
   }
   if (n_active == 1) return;
 
-  // The CTA that is last to finish for this (sequence, kv head) joins the splits.
-  __threadfence();
+  // The CTA that is last to finish for this (sequence, kv head) joins the splits.  One thread's fence behind the barrier covers
+  // what all have stored (and one behind the count what all will load): 128 fences cost the chain more.
   __syncthreads();
   if (tid == 0) {
+    __threadfence();
     const int old = atomicAdd(&counters[b * n_kv + kvh], 1);
     s_last = old == n_active - 1;
-    if (s_last) counters[b * n_kv + kvh] = 0;          // ready for the next launch
+    if (s_last) {
+      counters[b * n_kv + kvh] = 0;                    // ready for the next launch
+      __threadfence();
+    }
   }
   __syncthreads();
   if (!s_last) return;
-  __threadfence();
   // The splits' results come from L2, which answers slowly while the next product's CTAs fill their
   // rings: every thread issues all loads of a batch of splits for its two channels before it uses
   // any, and the (maximum, sum) pairs of the batch, which all channels of a head share, come into
