@@ -276,10 +276,10 @@ add_rmsnorm_vec_kernel(float *__restrict__ resid, const TD *__restrict__ delta, 
             t.z += d[j][p].z;
             t.w += d[j][p].w;
           }
-        v[j].x += (t.x + cb[j].x) * cs[j].x;
-        v[j].y += (t.y + cb[j].y) * cs[j].y;
-        v[j].z += (t.z + cb[j].z) * cs[j].z;
-        v[j].w += (t.w + cb[j].w) * cs[j].w;
+        v[j].x = fmaf(t.x + cb[j].x, cs[j].x, v[j].x);
+        v[j].y = fmaf(t.y + cb[j].y, cs[j].y, v[j].y);
+        v[j].z = fmaf(t.z + cb[j].z, cs[j].z, v[j].z);
+        v[j].w = fmaf(t.w + cb[j].w, cs[j].w, v[j].w);
       } else {
 #pragma unroll
         for (int p = 0; p < MAXP; ++p)
@@ -337,13 +337,13 @@ norm_rows_kernel(float *__restrict__ resid, const TD *__restrict__ delta, const 
       const int c4 = lane + j * 32;
       if (c4 < n4) {
         const float4 t = ld4(d + 4 * c4);
-        if (col_scale || col_bias) {
+        if (col_scale || col_bias) {         // spelled out, here and above: a compiler may or may not join the two by itself
           const float4 cs = col_scale ? ld4(col_scale + 4 * c4) : make_float4(1.f, 1.f, 1.f, 1.f);
           const float4 cb = col_bias ? ld4(col_bias + 4 * c4) : make_float4(0.f, 0.f, 0.f, 0.f);
-          v[j].x += (t.x + cb.x) * cs.x;
-          v[j].y += (t.y + cb.y) * cs.y;
-          v[j].z += (t.z + cb.z) * cs.z;
-          v[j].w += (t.w + cb.w) * cs.w;
+          v[j].x = fmaf(t.x + cb.x, cs.x, v[j].x);
+          v[j].y = fmaf(t.y + cb.y, cs.y, v[j].y);
+          v[j].z = fmaf(t.z + cb.z, cs.z, v[j].z);
+          v[j].w = fmaf(t.w + cb.w, cs.w, v[j].w);
         } else {
           v[j].x += t.x;
           v[j].y += t.y;
