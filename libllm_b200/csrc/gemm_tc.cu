@@ -393,6 +393,254 @@ int launch_tc(const void *x, long long ldx, const void *W, void *out, long long 
   return LLM_OK;
 }
 
+// ---------------------------------------------------------------- the gated unit of a prompt step, two SMs to a tile
+// At thousands of tokens a tile's operands, not its products, are what one SM cannot bring in fast enough: 256 rows of W x
+// 128 tokens need 48 KB per 64 of K, 94 bytes a cycle at the tensor cores' rate, and an SM's loads end at 64.  Here a
+// cluster of two CTAs works on one tile of 256 rows of W x 256 tokens (tcgen05 cta_group::2): each brings half of the
+// rows and half of the tokens, 32 KB for the same products, 64 bytes a cycle, and each holds the accumulator of its own 128 rows.
+// The CTA of even rank issues the products of both; its barriers count what both have loaded and read.
+//
+// A CTA's 128 rows are gate and up rows of 64 features in turns of 16 (one four-dimensional box of the map), so that the
+// epilogue's warps hold a feature's gate in lane l < 16 and its up in lane l + 16: the two trade every other
+// token by shuffles, each lane then has both values of 8 tokens in 16, and nothing passes through shared memory.
+// 2,048 tokens x [16,384, 2,048]: 118 us on one SM a tile, 92 here (1.49 PFLOP/s; the library product and its pass 136); 8,192 x
+// [28,672, 4,096]: 1,247 (the library's 1,544 + 215).
+constexpr int GP_FEATURES = 64;                // of one CTA; a pair has 128
+constexpr int GP_TOKENS = 256;                 // of the pair; each CTA loads 128
+constexpr int GP_HALF_BYTES = 128 * TC_BK * 2; // a CTA's rows, or its tokens, of one stage
+constexpr int GP_STAGES = 6;
+// Eight epilogue warps, two to a quarter of the lanes (128 tokens each): with four, the gated unit of a tile (an exponential, a
+// division, a shuffle and a store for each of 16,384 values) took longer than its products at K = 2,048 (115.7 us a launch at
+// 2,048 tokens instead of 92).
+constexpr int GP_THREADS = 64 + 256;
+constexpr size_t GP_SMEM = 1024 + (size_t)GP_STAGES * 2 * GP_HALF_BYTES + 256;
+
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned in_cta(unsigned addr, unsigned rank) {      // the same place in the shared memory of a CTA of the cluster
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename TO>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
+gated_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, TO *__restrict__ out, long long ldo,
+                  int M, int n_out, int K, int row_tiles, int tok_tiles, GluShape glu, int *status) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned long long *bars = (unsigned long long *)(smem + (size_t)GP_STAGES * 2 * GP_HALF_BYTES);
+  const unsigned bar_full = smem_u32(bars), bar_empty = smem_u32(bars + GP_STAGES);
+  const unsigned bar_tfull = smem_u32(bars + 2 * GP_STAGES), bar_tempty = smem_u32(bars + 2 * GP_STAGES + 2);
+  unsigned *tmem_slot = (unsigned *)(bars + 2 * GP_STAGES + 4);
+  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const unsigned rank = cluster_rank();
+  grid_dependents_launch();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < GP_STAGES; ++s) {
+      mbar_init(bar_full + 8 * s, 1);          // rank 0's: its loader, and the bytes of both
+      mbar_init(bar_empty + 8 * s, 1);         // each CTA's own: the products that read the stage, committed to both
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(bar_tfull + 8 * a, 1);         // each CTA's own
+      mbar_init(bar_tempty + 8 * a, 16);       // rank 0's: the epilogue warps of both
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tma_prefetch_map(&map_w);
+    tma_prefetch_map(&map_x);
+  }
+  if (warp == 1) {                             // in both CTAs: the pair's tensor memory is allocated together
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                              // both CTAs' barriers are there before anyone signals the other's
+  tc_fence_after();
+  const unsigned tmem_base = *tmem_slot;
+
+  const int n_tiles = row_tiles * tok_tiles, n_kblocks = (K + TC_BK - 1) / TC_BK;
+  const int first = blockIdx.x / 2, step = gridDim.x / 2;      // this pair's tiles
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ loader: this CTA's half of both operands
+    const bool leader = elect_one();
+    struct Walk {
+      int tile, kb;
+      bool valid;
+    };
+    auto next = [&](Walk &w) {
+      if (++w.kb >= n_kblocks) {
+        w.tile += step;
+        w.kb = 0;
+        w.valid = w.tile < n_tiles;
+      }
+    };
+    auto load_w = [&](const Walk &w, int stage) {
+      if (!leader) return;
+      const unsigned full = in_cta(bar_full + 8 * stage, 0);
+      if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, 4 * GP_HALF_BYTES);
+      const int group = ((w.tile / tok_tiles) * 2 + (int)rank) * (GP_FEATURES / 16);
+      asm volatile(
+          "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %3, %4}], [%5];"
+          ::"r"(smem_u32(smem + (size_t)stage * 2 * GP_HALF_BYTES)), "l"(&map_w), "r"(w.kb * TC_BK), "r"(0), "r"(group), "r"(full) : "memory");
+    };
+    auto load_x = [&](const Walk &w, int stage) {
+      if (!leader) return;
+      const unsigned full = in_cta(bar_full + 8 * stage, 0);
+      asm volatile(
+          "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+          ::"r"(smem_u32(smem + (size_t)stage * 2 * GP_HALF_BYTES) + GP_HALF_BYTES), "l"(&map_x), "r"(w.kb * TC_BK),
+          "r"(w.tile % tok_tiles * GP_TOKENS + (int)rank * 128), "r"(full) : "memory");
+    };
+    // weights before the dependency is waited for, tokens after it
+    Walk w{first, 0, first < n_tiles}, w2 = w;
+    int n_pre = 0;
+    for (; w.valid && n_pre < GP_STAGES; next(w), ++n_pre) load_w(w, n_pre);
+    grid_dependency_wait();
+    for (int s = 0; s < n_pre; ++s, next(w2)) load_x(w2, s);
+    int stage = n_pre % GP_STAGES;
+    unsigned phase = n_pre == GP_STAGES ? 1u : 0u;
+    bool ok = true;
+    for (; w.valid; next(w)) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, 1));
+      if (!ok) break;
+      load_w(w, stage);
+      load_x(w, stage);
+      if (++stage == GP_STAGES) {
+        stage = 0;
+        phase ^= 1;
+      }
+    }
+    if (!ok) {                                 // given up: what is in flight lands within this time, whoever's barrier it signals
+      const unsigned long long t0 = globaltimer();
+      while (globaltimer() - t0 < 2000000ull) {
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ products of both CTAs, issued by rank 0
+    const bool leader = elect_one();
+    constexpr unsigned IDESC = instr_desc(256, GP_TOKENS);
+    auto commit = [&](unsigned bar) {          // arrives at this barrier in both CTAs when the products so far are done
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                   ::"r"(bar), "h"((unsigned short)3) : "memory");
+    };
+    int stage = 0, iter = 0;
+    unsigned phase = 0;
+    bool ok = rank == 0;
+    for (int tile = first; tile < n_tiles && ok; tile += step, ++iter) {
+      const int acc = iter & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty + 8 * acc, ((iter >> 1) & 1) ^ 1, abort_flag, status, 2));
+      if (!ok) break;
+      tc_fence_after();
+      const unsigned d_tmem = tmem_base + acc * GP_TOKENS;
+      for (int kb = 0; kb < n_kblocks; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 3));
+        if (!ok) break;
+        tc_fence_after();
+        const unsigned a_addr = smem_u32(smem + (size_t)stage * 2 * GP_HALF_BYTES);
+        const unsigned long long a_desc = smem_desc(a_addr), b_desc = smem_desc(a_addr + GP_HALF_BYTES);
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < TC_BK / 16; ++kk)
+            asm volatile(
+                "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+                ::"r"(d_tmem), "l"(a_desc + (unsigned long long)(kk * 2)), "l"(b_desc + (unsigned long long)(kk * 2)), "r"(IDESC),
+                "r"(kk > 0 || kb > 0 ? 1u : 0u) : "memory");
+          commit(bar_empty + 8 * stage);
+        }
+        __syncwarp();
+        if (++stage == GP_STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+      if (ok && leader) commit(bar_tfull + 8 * acc);
+      __syncwarp();
+    }
+    grid_dependency_wait();
+  } else {
+    // ------------------------------------------------------------ epilogue of this CTA's 128 rows (warps 2..9)
+    grid_dependency_wait();
+    const int quarter = warp & 3, half = (warp - 2) / 4;       // the lanes of tensor memory the warp may read; its half of the tokens
+    constexpr int CHUNKS = GP_TOKENS / 32;
+    int iter = 0;
+    for (int tile = first; tile < n_tiles; tile += step, ++iter) {
+      const int acc = iter & 1, tok0 = tile % tok_tiles * GP_TOKENS + half * (GP_TOKENS / 2);
+      if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * acc, (iter >> 1) & 1, abort_flag, status, 4))) break;
+      tc_fence_after();
+      const int f = ((tile / tok_tiles) * 2 + (int)rank) * GP_FEATURES + quarter * 16 + (lane & 15);
+      const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * GP_TOKENS + half * (GP_TOKENS / 2));
+      float even[16], odd[16];
+      tc_ld16_issue(taddr, even);
+#pragma unroll 1
+      for (int c = 0; c < CHUNKS; c += 2) {
+        tc_ld_wait();
+        tc_ld_ready(even);
+        tc_ld16_issue(taddr + (c + 1) * 16, odd);
+        store_turns(even, out, ldo, f, n_out, tok0 + c * 16, M, glu);
+        tc_ld_wait();
+        tc_ld_ready(odd);
+        if (c + 2 < CHUNKS) tc_ld16_issue(taddr + (c + 2) * 16, even);
+        store_turns(odd, out, ldo, f, n_out, tok0 + (c + 1) * 16, M, glu);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_cta(bar_tempty + 8 * acc, 0)) : "memory");
+    }
+  }
+
+  // ---------------------------------------------------------------- teardown: neither CTA leaves while the other may signal it
+  tc_fence_before();
+  __syncwarp();
+  __syncthreads();
+  cluster_sync();
+  if (warp == 1) {
+    tc_fence_after();
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+template <typename TO>
+int launch_gated_pair(const void *x, long long ldx, const void *W, void *out, long long ldo, int M, int n_out, int K, const GluShape &glu,
+                      int *status, cudaStream_t stream) {
+  CUtensorMap map_w, map_x;
+  int rc = get_gated_map(W, n_out, K, &map_w);
+  if (rc != LLM_OK) return rc;
+  rc = get_map(x, M, K, ldx, 128, &map_x);
+  if (rc != LLM_OK) return rc;
+  const int row_tiles = (n_out + 2 * GP_FEATURES - 1) / (2 * GP_FEATURES), tok_tiles = (M + GP_TOKENS - 1) / GP_TOKENS;
+  const long long tiles = (long long)row_tiles * tok_tiles;
+  LLM_REQUIRE(tiles < (1ll << 30), "gemm_tc: too many tiles");
+  const int pairs = (int)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
+  auto kern = gated_pair_kernel<TO>;
+  LLM_CHECK_CUDA(llm_allow_smem(kern, GP_SMEM), "gemm_tc attribute");
+  LLM_CHECK_CUDA(llm_launch(kern, dim3(2 * pairs), dim3(GP_THREADS), GP_SMEM, stream, map_w, map_x, (TO *)out, ldo, M, n_out, K, row_tiles,
+                            tok_tiles, glu, status),
+                 "gemm_tc launch");
+  return LLM_OK;
+}
+
+// Whether the gated unit of M tokens and a stacked matrix of N rows runs two SMs to a tile: whole groups of 16 features (the map),
+// tiles for most pairs of SMs, and 512 tokens or more of which the last tile does not waste a fifth.  Measured against the library product and
+// its pass ([16,384, 2,048]): 300 tokens 45 us against 28, 512 34 against 40, 773 (of 1,024) 66 against 59, 1,024 56 against 72; with tiles for
+// half of the pairs ([2,048, 512], 1,024 tokens) 15 against 12.
+bool takes_pair(int M, int N) {
+  const long long tok_tiles = (M + GP_TOKENS - 1) / GP_TOKENS, row_tiles = (N / 2 + 2 * GP_FEATURES - 1) / (2 * GP_FEATURES);
+  return N % 32 == 0 && M >= 512 && tok_tiles * GP_TOKENS * 4 <= (long long)M * 5 && tok_tiles * row_tiles * 2 >= sm_count();
+}
+
 template <bool SWIGLU, typename TO>
 int dispatch_tc(const void *x, long long ldx, const void *W, void *out, long long ldo, int M, int N, int K, int k_parts,
                 long long part_stride, const GluShape &glu, int *status, cudaStream_t stream) {
@@ -406,6 +654,7 @@ int dispatch_tc(const void *x, long long ldx, const void *W, void *out, long lon
     if (M <= 16) TC_GO(16, 1);
     if (M <= 32) TC_GO(32, 1);
     if (M <= 64) TC_GO(64, 1);
+    if (takes_pair(M, N)) return launch_gated_pair<TO>(x, ldx, W, out, ldo, M, N / 2, K, glu, status, stream);
     TC_GO(128, 2);
   }
   if (M <= 16) TC_GO(16, 0);
@@ -438,6 +687,9 @@ LLM_EXPORT int llm_gemm_tc_suggest_parts(int M, int N, int K) {
   }
   return parts;
 }
+
+// 1 if the gated unit of these sizes runs two SMs to a tile.
+LLM_EXPORT int llm_gemm_tc_pairs(int M, int N) { return takes_pair(M, N); }
 
 // x [M, K] bfloat16 (row stride ldx elements), W [N, K] bfloat16 contiguous, out [M, N] of out_dtype,
 // or [M, N/2] with swiglu (W = stacked gate|up).  With k_parts > 1 (plain product, 32-bit out) part p

@@ -303,6 +303,10 @@ bool gemm_tc_supported(const Act &x, const Weight &w) {
   return x.dtype == DType::BF16 && w.dtype == DType::BF16 && x.rows > 0 && x.cols % 8 == 0 && (x.rows == 1 || x.ld % 8 == 0) &&
          (uintptr_t)x.data % 16 == 0 && (uintptr_t)w.data() % 16 == 0;
 }
+bool gemm_tc_pairs(const Act &x, const Weight &w) {
+  static auto f = resolve<int (*)(int, int)>("gemm_tc", "llm_gemm_tc_pairs");
+  return f((int)x.rows, (int)w.rows) != 0;
+}
 int gemm_tc_suggest_parts(int M, int N, int K) {
   static auto f = resolve<int (*)(int, int, int)>("gemm_tc", "llm_gemm_tc_suggest_parts");
   return f(M, N, K);

@@ -79,6 +79,7 @@ void random_fill(void *out, DType dtype, long long n, unsigned long long seed, i
 // ---- products
 void gemm_plain(const Act &x, const Weight &w, const float *bias, const Act &out, cudaStream_t s);
 bool gemm_tc_supported(const Act &x, const Weight &w);
+bool gemm_tc_pairs(const Act &x, const Weight &w);      // a gated unit of these sizes runs two SMs to a tile
 int gemm_tc_suggest_parts(int M, int N, int K);
 // The unit of a gated pair (gate g, up u): g' = min(g, limit), u' = clamp(u, -limit, limit), g' sigmoid(slope g') (u' + shift)
 struct Glu {

@@ -33,6 +33,7 @@ const FastSwitches &fast_switches() {
     f.moe_tc = !off("LIBLLM_B200_NO_MOE_TC");
     f.tc_tokens = num("LIBLLM_B200_TC_TOKENS", 256);
     f.fused_gate_up_tokens = num("LIBLLM_B200_FUSED_GATE_UP_TOKENS", 1024);
+    f.pair_gate_up_tokens = num("LIBLLM_B200_FUSED_GATE_UP_TOKENS", 0);
     f.gemv_tokens = num("LIBLLM_B200_GEMV_TOKENS", 0);
     return f;
   }();
@@ -173,10 +174,11 @@ Act fused_gated_linear(StepContext &ctx, const Act &x, const Weight &w, const ke
   Act m;
   if (x.dtype != DType::BF16) return m;
   m = small_batch_linear(ctx, x, w, ctx.dtype, true, false, glu);
-  // The gated unit of a prompt step in one launch of the tcgen05 product (two accumulators per
-  // tile), where that beats the library product followed by a pass of its own: measured at 2,048
-  // tokens, 129 us against 146 us at K = 2,048, but 403 us against 379 us at K = 4,096.
-  if (!m.data && f.gemm_tc && x.rows >= f.fused_gate_up_tokens && x.cols <= f.fused_gate_up_max_k && kernels::gemm_tc_supported(x, w)) {
+  // The gated unit of a prompt step in one launch of the tcgen05 product, where that beats the library product followed by a
+  // pass of its own: wherever the kernel takes two SMs to a tile (gemm_tc.cu: takes_pair), and with one SM to a tile (two accumulators)
+  // at 2,048 tokens 118 us against 136 at K = 2,048, but 403 against 387 at K = 4,096.
+  if (!m.data && f.gemm_tc && kernels::gemm_tc_supported(x, w) &&
+      (kernels::gemm_tc_pairs(x, w) ? x.rows >= f.pair_gate_up_tokens : x.rows >= f.fused_gate_up_tokens && x.cols <= f.fused_gate_up_max_k)) {
     m = ctx.arena->act(ctx.dtype, x.rows, w.rows / 2);
     flush_chain(ctx);
     kernels::gemm_tc(x, w, m, true, ctx.tc_status, ctx.stream, glu ? *glu : kernels::Glu());

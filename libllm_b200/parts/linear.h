@@ -21,6 +21,7 @@ struct FastSwitches {
   int tc_tokens = 256;                 // steps of up to this many tokens take the tcgen05 product
   int fused_gate_up_tokens = 1024;     // prompt steps from this many tokens fuse SwiGLU into the product ...
   int fused_gate_up_max_k = 3072;      // ... when the width is at most this
+  int pair_gate_up_tokens = 0;         // the same where the kernel takes two SMs to a tile (whatever the width)
   int gemv_tokens = 0;                 // steps of up to this many tokens take the mma.sync weight streamer
 };
 const FastSwitches &fast_switches();
