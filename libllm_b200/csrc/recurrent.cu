@@ -205,69 +205,81 @@ LLM_EXPORT int llm_causal_conv(int dtype, const void *h, long long ldh, void *ou
 constexpr int DP_WARPS = 4;
 constexpr int DP_TOKENS = 32;                        // tokens of a CTA
 
+// DP_TT tokens to a warp at a time: what bounds it is reading W2's rows from shared memory, a read to a multiplication with one
+// token and three to eight with four (168 -> 104 us for 2,841 tokens of 32 heads of 64, rank 64).  One where a decay input is too wide for four.
+template <int DP_TT>
 __global__ void __launch_bounds__(DP_WARPS * 32)
 delta_prepare_kernel(const float *__restrict__ proj, long long ld, int off_k, int off_a, int off_x1, int rank,
                      const float *__restrict__ w2, const float *__restrict__ w0, const float *__restrict__ a_bias,
                      float decay_scale, float key_eps, int n_tokens, int n_heads, int d, int w2_shared,
                      float *__restrict__ prep) {
-  extern __shared__ float dp_smem[];                 // tanh(x1) [warps][rank], then W2's rows of the head [d][rank + 1]
+  extern __shared__ float dp_smem[];                 // tanh(x1) [warps][rank][DP_TT], then W2's rows of the head [d][rank + 1]
   grid_dependents_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int hd = blockIdx.y;
-  float *th = dp_smem + warp * rank;
-  float *w2s = dp_smem + DP_WARPS * rank;
+  float *th = dp_smem + warp * rank * DP_TT;
+  float *w2s = dp_smem + DP_WARPS * rank * DP_TT;
   const float *w2h = w2 + (size_t)hd * d * rank;
   if (w2_shared)                                     // weights: nothing of the step is read yet
     for (int i = threadIdx.x; i < d * rank; i += DP_WARPS * 32) w2s[(i / rank) * (rank + 1) + i % rank] = w2h[i];
   grid_dependency_wait();
   __syncthreads();
   const int t1 = min(n_tokens, (int)(blockIdx.x + 1) * DP_TOKENS);
-  for (int t = blockIdx.x * DP_TOKENS + warp; t < t1; t += DP_WARPS) {
-    const float *row = proj + (size_t)t * ld;
-    const float *k = row + off_k + (size_t)hd * d;
+  for (int t = blockIdx.x * DP_TOKENS + warp * DP_TT; t < t1; t += DP_WARPS * DP_TT) {
+    const int nt = min(DP_TT, t1 - t);
     __syncwarp();
-    for (int q = lane; q < rank; q += 32) th[q] = tanhf(row[off_x1 + q]);
-    float ss = 0.f;
-    for (int i = lane; i < d; i += 32) ss = fmaf(k[i], k[i], ss);
-    ss = warp_sum(ss);
+    for (int q = lane; q < rank; q += 32)
+#pragma unroll
+      for (int u = 0; u < DP_TT; ++u) th[q * DP_TT + u] = u < nt ? tanhf(proj[(size_t)(t + u) * ld + off_x1 + q]) : 0.f;
+    float inv[DP_TT];
+#pragma unroll
+    for (int u = 0; u < DP_TT; ++u) {
+      const float *k = proj + (size_t)(t + min(u, nt - 1)) * ld + off_k + (size_t)hd * d;
+      float ss = 0.f;
+      for (int i = lane; i < d; i += 32) ss = fmaf(k[i], k[i], ss);
+      inv[u] = 1.f / sqrtf(warp_sum(ss) + key_eps);
+    }
     __syncwarp();
-    const float inv = 1.f / sqrtf(ss + key_eps);
-    float *o = prep + ((size_t)t * n_heads + hd) * 3 * d;
-    for (int i0 = 0; i0 < d; i0 += 128) {             // four channels of a lane at a time: four chains of sums, not one
-      float z[4];
-      int chs[4];
+    for (int i0 = 0; i0 < d; i0 += 64) {              // two channels of a lane for each of the tokens
+      float z[DP_TT][2];
+      const int ch0 = min(i0 + lane, d - 1), ch1 = min(i0 + lane + 32, d - 1);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int i = i0 + lane + 32 * c;
-        chs[c] = i < d ? i : -1;
-        z[c] = i < d ? w0[hd * d + i] : 0.f;
+      for (int u = 0; u < DP_TT; ++u) {
+        z[u][0] = w0[hd * d + ch0];
+        z[u][1] = w0[hd * d + ch1];
       }
-      if (w2_shared) {
-        for (int q = 0; q < rank; ++q) {
-          const float tq = th[q];
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (chs[c] >= 0) z[c] = fmaf(w2s[chs[c] * (rank + 1) + q], tq, z[c]);
+      const float *r0 = w2_shared ? w2s + ch0 * (rank + 1) : w2h + (size_t)ch0 * rank, *r1 = w2_shared ? w2s + ch1 * (rank + 1) : w2h + (size_t)ch1 * rank;
+#pragma unroll 4
+      for (int q = 0; q < rank; ++q) {
+        float tq[DP_TT];
+        if constexpr (DP_TT == 4) {
+          const float4 v = ld4(th + q * DP_TT);
+          tq[0] = v.x, tq[1] = v.y, tq[2] = v.z, tq[3] = v.w;
+        } else {
+          tq[0] = th[q];
         }
-      } else {
-        for (int q = 0; q < rank; ++q) {
-          const float tq = th[q];
+        const float a0 = r0[q], a1 = r1[q];
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (chs[c] >= 0) z[c] = fmaf(w2h[(size_t)chs[c] * rank + q], tq, z[c]);
+        for (int u = 0; u < DP_TT; ++u) {
+          z[u][0] = fmaf(a0, tq[u], z[u][0]);
+          z[u][1] = fmaf(a1, tq[u], z[u][1]);
         }
       }
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int i = chs[c];
-        if (i < 0) continue;
-        const int ch = hd * d + i;
-        const float u = k[i] * inv;
-        const float a = 1.f / (1.f + expf(-(row[off_a + ch] + a_bias[ch])));
-        o[i] = expf(-decay_scale / (1.f + expf(-z[c])));
-        o[d + i] = a * u;
-        o[2 * d + i] = u;
-      }
+      for (int u = 0; u < DP_TT; ++u)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int i = i0 + lane + 32 * c;
+          if (i >= d || u >= nt) continue;
+          const int ch = hd * d + i;
+          const float *row = proj + (size_t)(t + u) * ld;
+          const float x = row[off_k + ch] * inv[u];
+          const float a = 1.f / (1.f + expf(-(row[off_a + ch] + a_bias[ch])));
+          float *o = prep + ((size_t)(t + u) * n_heads + hd) * 3 * d;
+          o[i] = expf(-decay_scale / (1.f + expf(-z[u][c])));
+          o[d + i] = a * x;
+          o[2 * d + i] = x;
+        }
     }
   }
 }
@@ -489,12 +501,15 @@ LLM_EXPORT int llm_delta_rule(const float *proj, long long ld, int off_r, int of
   LLM_REQUIRE(d <= 256, "delta_rule: heads of %d channels are not supported (up to 256)", d);
   LLM_REQUIRE(n_heads <= 65535 && n_seqs < 2147483647, "delta_rule: too many heads or sequences");
   {
-    const size_t with_w2 = ((size_t)DP_WARPS * rank + (size_t)d * (rank + 1)) * sizeof(float);
-    const int w2_shared = with_w2 <= 96 * 1024;
-    const size_t smem = w2_shared ? with_w2 : (size_t)DP_WARPS * rank * sizeof(float);
-    LLM_REQUIRE(smem <= 96 * 1024, "delta_rule: a decay input of rank %d is not supported", rank);
-    LLM_CHECK_CUDA(llm_allow_smem(delta_prepare_kernel, smem), "delta_prepare attribute");
-    llm_launch(delta_prepare_kernel, dim3((unsigned)((n_tokens + DP_TOKENS - 1) / DP_TOKENS), n_heads), dim3(DP_WARPS * 32), smem, stream,
+    auto bytes = [&](int tt, bool with_w2) { return ((size_t)DP_WARPS * rank * tt + (with_w2 ? (size_t)d * (rank + 1) : 0)) * sizeof(float); };
+    constexpr size_t MOST = 96 * 1024;
+    const int tt = bytes(4, true) <= MOST || (bytes(1, true) > MOST && bytes(4, false) <= MOST) ? 4 : 1;
+    const int w2_shared = bytes(tt, true) <= MOST;
+    const size_t smem = bytes(tt, w2_shared);
+    LLM_REQUIRE(smem <= MOST, "delta_rule: a decay input of rank %d is not supported", rank);
+    auto kern = tt == 4 ? delta_prepare_kernel<4> : delta_prepare_kernel<1>;
+    LLM_CHECK_CUDA(llm_allow_smem(kern, smem), "delta_prepare attribute");
+    llm_launch(kern, dim3((unsigned)((n_tokens + DP_TOKENS - 1) / DP_TOKENS), n_heads), dim3(DP_WARPS * 32), smem, stream,
                proj, ld, off_k, off_a, off_x1, rank, w2, w0, a_bias, decay_scale, key_eps, n_tokens, n_heads, d, w2_shared, prep);
     LLM_CHECK_LAUNCH("delta_prepare");
   }

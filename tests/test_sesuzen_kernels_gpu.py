@@ -266,7 +266,7 @@ def delta_reference(proj, w2, w0, ab, H, d, rank, S=None):
     return P.delta_scan(r, k, v, decay, rate, unit, S)
 
 
-@pytest.mark.parametrize("H,d,rank", [(2, 16, 8), (3, 24, 5), (1, 128, 24), (5, 8, 3), (2, 64, 16), (1, 200, 9), (2, 32, 1)])
+@pytest.mark.parametrize("H,d,rank", [(2, 16, 8), (3, 24, 5), (1, 128, 24), (5, 8, 3), (2, 64, 16), (1, 200, 9), (2, 32, 1), (1, 64, 97), (1, 16, 1700)])
 def test_delta_rule_with_carried_state(H, d, rank):
     """Two sequences in slots that are not in order, each brought in two steps (a long one and single tokens beside a
     prompt): the state written by one launch is what the next one starts from."""
