@@ -299,6 +299,38 @@ def test_delta_rule_with_carried_state(H, d, rank):
     assert float(state[[0, 2]].abs().max()) == 0
 
 
+# heads as wide as the tile, narrower and the wider tile; runs that end with 1, 15 and 16 tokens, and a sequence of one run
+@pytest.mark.parametrize("H,d,rank", [(2, 64, 8), (1, 128, 5), (3, 20, 4), (1, 100, 9)])
+def test_delta_rule_sixteen_tokens_at_a_time(H, d, rank):
+    """Three prompts from states that are not zero, in slots out of order, behind an earlier step: against the plain recurrence, and
+    beside the token-by-token kernel on the same inputs: no farther from 64 bits than that by more than one rounding of the result."""
+    from libllm_b200.csrc import ops
+    g = torch.Generator().manual_seed(H * d + rank)
+    lens = [33, 16, 127]
+    data = [delta_inputs(n, H, d, rank, g) for n in lens]
+    w2, w0, ab = data[0][1:]
+    W = H * d
+    i32 = dict(dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 1, 0], **i32)
+    start = torch.tensor([0, 33, 49, 176], **i32)
+    begin = torch.randn(4, H, d, d, generator=g) * 0.3
+    proj = torch.cat([x[0] for x in data]).to(DEV)
+    got = {}
+    for chunks in (False, True):
+        state = begin.clone().to(DEV)
+        out = ops.delta_rule(proj, (0, W, 2 * W, 4 * W, 5 * W), rank, w2.to(DEV), w0.to(DEV), ab.to(DEV), P.DECAY_SCALE, P.KEY_EPS, state, start,
+                             slots, H, d, in_chunks=chunks)
+        got[chunks] = out.cpu().double(), state.cpu().double()
+        assert torch.equal(state[2].cpu(), begin[2])
+    for b, n in enumerate(lens):
+        o0 = int(start[b])
+        ref_o, ref_S = delta_reference(data[b][0], w2, w0, ab, H, d, rank, begin[int(slots[b])].double().transpose(1, 2))
+        off = {c: (float((got[c][0][o0:o0 + n].view(n, H, d) - ref_o).norm() / ref_o.norm()),
+                   float((got[c][1][int(slots[b])].transpose(1, 2) - ref_S).norm() / ref_S.norm())) for c in got}
+        for one, many in zip(off[False], off[True]):
+            assert many <= one + 2 ** -24, (b, off)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,dv", [(3, 24), (2, 64), (5, 8), (1, 200)])
 def test_norm_per_head_weight_and_gate(dtype, H, dv):
