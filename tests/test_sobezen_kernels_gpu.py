@@ -251,3 +251,25 @@ def test_queries_take_in_the_keys_matrix_and_results_are_expanded(T, H, d, rot, 
     ref = torch.einsum("thc,hjc->thj", x3, v3)
     room = (R / 32 + 8) * 2 ** -24 * torch.einsum("thc,hjc->thj", x3.abs(), v3.abs()) + result * ref.abs()
     assert bool(((y.cpu().double().view(T, H, dv) - ref).abs() <= room).all())
+
+
+# ranks on either side of the sixteen values a thread holds, CTAs whose channels begin inside a head and end in another key head's
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H,G,d,dv,ranks", [(6, 2, 50, 44, (16, 17)), (5, 5, 96, 64, (40, 3)), (8, 1, 64, 80, (15, 33))])
+def test_channel_delta_with_ranks_and_heads_beside_a_threads_share(H, G, d, dv, ranks, dtype):
+    """Prompts, portions and single tokens of the gated delta rule, state carried in slots out of order."""
+    m, w, _ = mixer_of([S.layer(S.delta(H, G, d, dv, 3), None)], 0, dtype, 21, ranks)
+    sizes = dict(heads=H, kv_heads=G, dim=d, vdim=dv)
+    lens = [70, 9]
+    x = sharp_inputs(22, lens)
+    kept = {n["name"]: (torch.zeros([4, *n["shape"]], dtype=DT[n["dtype"]], device=DEV), n) for n in m.description["state"]}
+    state = [dict(name=k, ptr=t.data_ptr(), shape=n["shape"], dtype=n["dtype"], n_slots=4) for k, (t, n) in kept.items()]
+    got = run_in_portions([m], [None], x, [[33, 1], [1, 1], [35, 6], [1, 1]], dtype, lens, state=state, slots=[2, 0])
+    for b in range(2):
+        survives = []
+        ref = P.channel_delta(w, "l0.mix.", sizes, x[b].double(), EPS, survives)
+        # a head's norm divides by the head: rows where one all but cancels hang on the roundings of its 16-bit inputs
+        clear = survives[0] > (0.0 if dtype == "float32" else 0.1 * float(survives[0].mean()))
+        e = (got[0][b].double() - ref).norm(dim=-1) / ref.norm(dim=-1).mean()
+        assert int(clear.sum()) > len(ref) // 2
+        assert float(e[clear].max()) < (1e-4 if dtype == "float32" else 16 * 2 ** -8), (b, float(e[clear].max()))
