@@ -344,6 +344,23 @@ def test_attention_decode(n_heads, n_kv, d, window, chunk, n_splits):
         close(out[b].view(1, n_heads, d), ref, "bfloat16", scale=1.0)
 
 
+# runs of keys beside the eight asked for together and the 64 whose weights lie in shared memory; one to two channels a thread
+@pytest.mark.parametrize("n_heads,n_kv,d", [(2, 1, 16), (4, 1, 64), (1, 1, 128)])
+def test_many_runs_of_keys_are_joined(n_heads, n_kv, d):
+    from libllm_b200.csrc import ops
+    lens, page, n_splits = [511, 512, 513, 4095, 4096, 4097, 4500], 64, 72
+    B = len(lens)
+    K, V, table, ks, vs = paged_cache(B, lens, n_kv, d, page, "bfloat16", 27)
+    q = rnd((B, n_heads * d), "bfloat16", 28)
+    pos = torch.tensor([l - 1 for l in lens], dtype=torch.int32, device=DEV)
+    out = torch.empty((B, n_heads * d), dtype=torch.bfloat16, device=DEV)
+    ws_o, ws_ml = (torch.full((B * n_heads * n_splits * w,), float("nan"), device=DEV) for w in (d, 2))
+    ops.attention_decode(q, out, K, V, pos, table, n_heads, n_kv, d, page, 64, n_splits, None, 1 / math.sqrt(d), ws_o, ws_ml)
+    for b in range(B):
+        ref = P.attention_scores_softmax_values(q[b:b + 1].cpu().view(1, n_heads, d), ks[b], vs[b], None)
+        close(out[b].view(1, n_heads, d), ref, "bfloat16", scale=1.0)
+
+
 def prefill_inputs(lens, q_lens):
     start = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32, device=DEV)
     past = torch.tensor([l - n for l, n in zip(lens, q_lens)], dtype=torch.int32, device=DEV)
