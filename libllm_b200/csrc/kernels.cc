@@ -730,11 +730,11 @@ void moe_identity(const Act &x, const int *chosen, const float *weight, int n_ex
 LLM_KERNEL("recurrent", llm_causal_conv_mode, int, const void *, long long, void *, long long, const float *, void *, const int *,
            const int *, const int *, const int *, const int *, int, int, int, int, int, int, cudaStream_t)
 LLM_KERNEL("recurrent", llm_delta_scan, const float *, long long, int, int, int, const float *, float *, float *, long long, const int *,
-           const int *, int, int, int, int, int, float *, cudaStream_t)
+           const int *, int, int, int, int, int, cudaStream_t)
 LLM_KERNEL("recurrent", llm_channel_delta_prepare, float *, long long, const float *, long long, int, int, int, int, int, const float *,
            const float *, const float *, const float *, float, float *, float *, int, int, int, int, int, cudaStream_t)
 LLM_KERNEL("recurrent", llm_delta_rule, const float *, long long, int, int, int, int, int, int, const float *, const float *,
-           const float *, float, float, float *, float *, float *, long long, const int *, const int *, int, int, int, int, float *, cudaStream_t)
+           const float *, float, float, float *, float *, float *, long long, const int *, const int *, int, int, int, int, cudaStream_t)
 LLM_KERNEL("recurrent", llm_head_norm_gate, const float *, long long, const float *, const float *, long long, float, int, int, int,
            void *, int, long long, cudaStream_t)
 void causal_conv(const Act &h, const Act &out, const float *weight, void *state, const int *tok_seq, const int *tok_pos,
@@ -745,10 +745,10 @@ void causal_conv(const Act &h, const Act &out, const float *weight, void *state,
            tok_pos, seq_start, seq_past, seq_slot, (int)h.rows, n_seqs, (int)h.cols, taps, single_tokens ? 1 : 0, silu_alone ? 1 : 0, s);
 }
 void delta_scan(const Act &rows, int off_r, int off_k, int off_v, const float *prep, float *state, const Act &out, const int *seq_start,
-                const int *seq_slot, int n_seqs, int n_heads, int d, int dv, float *records, cudaStream_t s) {
+                const int *seq_slot, int n_seqs, int n_heads, int d, int dv, cudaStream_t s) {
   if (rows.dtype != DType::F32 || out.dtype != DType::F32) LLM_THROW(InvalidArg, "delta_scan: vectors and results are 32-bit");
   LLM_CALL("recurrent", llm_delta_scan, (const float *)rows.data, (long long)rows.ld, off_r, off_k, off_v, prep, state, (float *)out.data,
-           (long long)out.ld, seq_start, seq_slot, (int)rows.rows, n_seqs, n_heads, d, dv, records, s);
+           (long long)out.ld, seq_start, seq_slot, (int)rows.rows, n_seqs, n_heads, d, dv, s);
 }
 void channel_delta_prepare(const Act &cv, const Act &proj, int off_b, int off_a1, int rank_a, int off_g1, int rank_g, const float *a2,
                            const float *dt_bias, const float *a_log, const float *g2, float key_eps, float *prep, float *gate,
@@ -759,15 +759,11 @@ void channel_delta_prepare(const Act &cv, const Act &proj, int off_b, int off_a1
 }
 void delta_rule(const Act &proj, int off_r, int off_k, int off_v, int off_a, int off_x1, int rank, const float *w2, const float *w0,
                 const float *a_bias, float decay_scale, float key_eps, float *prep, float *state, const Act &out,
-                const int *seq_start, const int *seq_slot, int n_seqs, int n_heads, int d, float *records, cudaStream_t s) {
+                const int *seq_start, const int *seq_slot, int n_seqs, int n_heads, int d, cudaStream_t s) {
   if (proj.dtype != DType::F32 || out.dtype != DType::F32) LLM_THROW(InvalidArg, "delta_rule: projections and results are 32-bit");
   LLM_CALL("recurrent", llm_delta_rule, (const float *)proj.data, (long long)proj.ld, off_r, off_k, off_v, off_a, off_x1, rank, w2, w0,
            a_bias, decay_scale, key_eps, prep, state, (float *)out.data, (long long)out.ld, seq_start, seq_slot, (int)proj.rows,
-           n_seqs, n_heads, d, records, s);
-}
-size_t delta_chunk_floats(int n_tokens, int n_seqs, int n_heads, int d) {
-  static auto f = resolve<long long (*)(int, int, int, int)>("recurrent", "llm_delta_chunk_floats");
-  return (size_t)f(n_tokens, n_seqs, n_heads, d);
+           n_seqs, n_heads, d, s);
 }
 LLM_KERNEL("recurrent", llm_delta_step, const float *, long long, int, int, int, int, int, int, int, const float *, const float *,
            const float *, float, float, const float *, float, float *, void *, int, long long, const int *, int, int, int, cudaStream_t)

@@ -292,9 +292,7 @@ void causal_conv(const Act &h, const Act &out, const float *weight, void *state,
 // The delta rule's recurrence alone: rows (32-bit) hold r, k (heads x d) and v (heads x dv) at their offsets, prep
 // [tokens, heads, 3, d] the decay w, the removal b and the direction u; state [slots, heads, dv, d]; out [tokens, heads * dv].
 void delta_scan(const Act &rows, int off_r, int off_k, int off_v, const float *prep, float *state, const Act &out, const int *seq_start,
-                const int *seq_slot, int n_seqs, int n_heads, int d, int dv, float *records, cudaStream_t s);
-// Floats of `records`, the scratch with which both recurrences take a prompt's tokens sixteen at a time; 0: they take none (null).
-size_t delta_chunk_floats(int n_tokens, int n_seqs, int n_heads, int d);
+                const int *seq_slot, int n_seqs, int n_heads, int d, int dv, cudaStream_t s);
 // The gated delta rule's vectors from the convolved projections (csrc/recurrent.cu says which).
 void channel_delta_prepare(const Act &cv, const Act &proj, int off_b, int off_a1, int rank_a, int off_g1, int rank_g, const float *a2,
                            const float *dt_bias, const float *a_log, const float *g2, float key_eps, float *prep, float *gate,
@@ -303,7 +301,7 @@ void channel_delta_prepare(const Act &cv, const Act &proj, int off_b, int off_a1
 // input within a row); prep: scratch [tokens, heads, 3, d] floats; state [slots, heads, d, d] floats; out [tokens, heads * d].
 void delta_rule(const Act &proj, int off_r, int off_k, int off_v, int off_a, int off_x1, int rank, const float *w2, const float *w0,
                 const float *a_bias, float decay_scale, float key_eps, float *prep, float *state, const Act &out,
-                const int *seq_start, const int *seq_slot, int n_seqs, int n_heads, int d, float *records, cudaStream_t s);
+                const int *seq_start, const int *seq_slot, int n_seqs, int n_heads, int d, cudaStream_t s);
 // A step of single tokens (row b = sequence b): the same, with the norm over each head, its weight and the gate
 // (logits at off_g of the rows) behind it, in one launch; out [sequences, heads * d] in the engine's type.
 bool delta_step_supported(int d);

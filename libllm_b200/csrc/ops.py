@@ -684,29 +684,21 @@ def causal_conv(h: torch.Tensor, out: torch.Tensor, weight: torch.Tensor, state:
 
 def delta_rule(proj: torch.Tensor, offsets, rank: int, w2: torch.Tensor, w0: torch.Tensor, a_bias: torch.Tensor,
                decay_scale: float, key_eps: float, state: torch.Tensor, seq_start: torch.Tensor, seq_slot: torch.Tensor,
-               n_heads: int, d: int, in_chunks: bool = False) -> torch.Tensor:
+               n_heads: int, d: int) -> torch.Tensor:
     """The generalized delta rule over 32-bit rows ``proj`` ([T, >= ...]; ``offsets`` of r, k, v, the removal logits and
-    the decay's low-rank input); state [slots, heads, d, d] (a column's rows together) is moved on.  Returns o [T, heads * d].  ``in_chunks``:
-    sixteen tokens at a time (the call must be of a shape that is taken so)."""
+    the decay's low-rank input); state [slots, heads, d, d] (a column's rows together) is moved on.  Returns o [T, heads * d]."""
     _on_gpu(proj, w2, w0, a_bias, state, seq_start, seq_slot)
     T = proj.shape[0]
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and state.dtype == torch.float32 and state.is_contiguous()
     prep = torch.empty(T, n_heads, 3, d, dtype=torch.float32, device=proj.device)
     out = torch.empty(T, n_heads * d, dtype=torch.float32, device=proj.device)
     off_r, off_k, off_v, off_a, off_x1 = offsets
-    records = None
-    if in_chunks:
-        f = build.load("recurrent").llm_delta_chunk_floats
-        f.argtypes, f.restype = [c_int] * 4, c_longlong
-        n = f(T, seq_slot.numel(), n_heads, d)
-        assert n > 0, "this shape goes token by token"
-        records = torch.full((n,), float("nan"), dtype=torch.float32, device=proj.device)
     _call("recurrent", "llm_delta_rule",
           [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float, c_void_p,
-           c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+           c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
           _ptr(proj), proj.stride(0), off_r, off_k, off_v, off_a, off_x1, rank, _ptr(w2), _ptr(w0), _ptr(a_bias), float(decay_scale),
           float(key_eps), _ptr(prep), _ptr(state), _ptr(out), out.stride(0), _ptr(seq_start), _ptr(seq_slot), T,
-          seq_slot.numel(), n_heads, d, _ptr(records), _stream())
+          seq_slot.numel(), n_heads, d, _stream())
     return out
 
 

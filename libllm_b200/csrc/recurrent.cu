@@ -499,382 +499,10 @@ static int launch_delta_scan(const float *proj, long long ld, int off_r, int off
   return LLM_OK;
 }
 
-// ---------------------------------------------------------------- the recurrence of a prompt, sixteen tokens at a time
-// delta_rule_kernel walks a prompt token by token, and each token waits for the one before: 262 ns a token.  With S0 the state before a run of tokens 1 .. C, W_i the product of the first i decays and D_{j,i} the
-// product of the decays j + 1 .. i (elementwise; only products, nothing is divided, so decays of nought are fine),
-//   S_i   = W_i S0 + sum_{j <= i} D_{j,i} (k_j v_j^T - b_j x_j^T),      x_i = u_i^T S_{i-1}  (what the removal reads),
-//   x_i   = (W_{i-1} u_i)^T S0 + sum_{j < i} (A_ij v_j - B_ij x_j),     A_ij = u_i . D_{j,i-1} k_j,  B_ij = u_i . D_{j,i-1} b_j,
-//   o_i   = (W_i r_i)^T S0 + sum_{j <= i} (E_ij v_j - F_ij x_j),        E_ij = r_i . D_{j,i} k_j,    F_ij = r_i . D_{j,i} b_j,
-// so that everything but S0 is known without the recurrence: delta_chunks_kernel works it out for all runs of all sequences at once,
-// with the unit triangular system (I + B) x = W u S0 + A v solved once for all columns (T = (I + B)^-1, M = T A), and
-// delta_chunk_scan_kernel goes from run to run with four small products.  All 32-bit, and no
-// farther from 64 bits than token by token (a test holds them side by side).  32 heads of 64, two prompts of 2,000 and 841 tokens: 536 -> 113 +
-// 252 us.
-constexpr int DC = 16;                         // tokens of a run
-constexpr int DC_THREADS = 128;
-// A run's record, floats: [16][D] each of W u, W r, D k, D b (the latter two to the run's end), [D] decays of the whole run, then T, M, E, F in
-// pieces of four columns ([4][16 rows][4]) so that sixteen rows' pieces lie side by side.
-__host__ __device__ constexpr int delta_record(int D) { return 64 * D + D + 4 * DC * DC; }
-
-// The run with number `id` among all sequences' runs: its sequence and its place there, or false.
-__device__ __forceinline__ bool find_run(const int *__restrict__ seq_start, int n_seqs, int id, int *b, int *run) {
-  for (int s = 0; s < n_seqs; ++s) {
-    const int runs = (seq_start[s + 1] - seq_start[s] + DC - 1) / DC;
-    if (id < runs) {
-      *b = s;
-      *run = id;
-      return true;
-    }
-    id -= runs;
-  }
-  return false;
-}
-
-template <int D>
-__global__ void __launch_bounds__(DC_THREADS)
-delta_chunks_kernel(const float *__restrict__ proj, long long ld, int off_r, int off_k, const float *__restrict__ prep,
-                    const int *__restrict__ seq_start, int n_seqs, int n_heads, int d, float *__restrict__ records) {
-  constexpr int Q = D / 32;
-  extern __shared__ float ck_sm[];             // w, b, u, k, r [16][D]; A, B, E, F, T [16][17]
-  float *sw = ck_sm, *sb = sw + DC * D, *su = sb + DC * D, *sk = su + DC * D, *sr = sk + DC * D;
-  constexpr int LM = DC + 1;
-  float *mA = sr + DC * D, *mB = mA + DC * LM, *mE = mB + DC * LM, *mF = mE + DC * LM, *mT = mF + DC * LM;
-  grid_dependents_launch();
-  grid_dependency_wait();
-  int b, run;
-  if (!find_run(seq_start, n_seqs, blockIdx.x, &b, &run)) return;
-  const int hd = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = seq_start[b] + run * DC, nt = min(DC, seq_start[b + 1] - t0);
-#pragma unroll 4
-  for (int e = tid; e < DC * D; e += DC_THREADS) {
-    const int t = e / D, c = e % D;
-    const bool in = t < nt && c < d;
-    const float *row = proj + (size_t)(t0 + (in ? t : 0)) * ld + (size_t)hd * d + (in ? c : 0);
-    const float *pr = prep + ((size_t)(t0 + (in ? t : 0)) * n_heads + hd) * 3 * d + (in ? c : 0);
-    sw[e] = in ? pr[0] : 1.f;
-    sb[e] = in ? pr[d] : 0.f;
-    su[e] = in ? pr[2 * d] : 0.f;
-    sk[e] = in ? row[off_k] : 0.f;
-    sr[e] = in ? row[off_r] : 0.f;
-  }
-  for (int e = tid; e < 4 * DC * LM; e += DC_THREADS) mA[e] = 0.f;
-  __syncthreads();
-  float *rec = records + ((size_t)blockIdx.x * n_heads + hd) * delta_record(D);
-  // decays from the run's beginning and to its end
-  for (int c = tid; c < D; c += DC_THREADS) {
-    float w = 1.f;
-#pragma unroll
-    for (int t = 0; t < DC; ++t) {
-      rec[t * D + c] = su[t * D + c] * w;
-      w *= sw[t * D + c];
-      rec[(DC + t) * D + c] = sr[t * D + c] * w;
-    }
-    rec[4 * DC * D + c] = w;
-    w = 1.f;
-#pragma unroll
-    for (int t = DC - 1; t >= 0; --t) {
-      rec[(2 * DC + t) * D + c] = sk[t * D + c] * w;
-      rec[(3 * DC + t) * D + c] = sb[t * D + c] * w;
-      w *= sw[t * D + c];
-    }
-  }
-  // pairs: a warp takes four tokens j (as many pairs as any other warp) and carries their k and b, decaying, along the later ones
-  for (int n = 0; n < 4; ++n) {
-    const int j = n == 0 ? warp : n == 1 ? 7 - warp : n == 2 ? 8 + warp : 15 - warp;
-    float qk[Q], qb[Q];
-    float e0 = 0.f, f0 = 0.f;
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int c = j * D + lane + 32 * q;
-      qk[q] = sk[c];
-      qb[q] = sb[c];
-      e0 = fmaf(sr[c], qk[q], e0);
-      f0 = fmaf(sr[c], qb[q], f0);
-    }
-    e0 = warp_sum(e0);
-    f0 = warp_sum(f0);
-    if (lane == 0) {
-      mE[j * LM + j] = e0;
-      mF[j * LM + j] = f0;
-    }
-    for (int i = j + 1; i < DC; ++i) {
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        const int c = i * D + lane + 32 * q;
-        v[0] = fmaf(su[c], qk[q], v[0]);
-        v[1] = fmaf(su[c], qb[q], v[1]);
-        qk[q] *= sw[c];
-        qb[q] *= sw[c];
-        v[2] = fmaf(sr[c], qk[q], v[2]);
-        v[3] = fmaf(sr[c], qb[q], v[3]);
-      }
-      // four sums over the lanes: half of the values go to half of the lanes, twice
-      const bool hi = lane & 16;
-      float x0 = hi ? v[2] : v[0], x1 = hi ? v[3] : v[1];
-      x0 += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
-      x1 += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
-      const bool odd = lane & 8;
-      float x = odd ? x1 : x0;
-      x += __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 8);
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if ((lane & 7) == 0) {                   // lanes 0, 8, 16, 24: A, B, E, F
-        float *m = lane == 0 ? mA : lane == 8 ? mB : lane == 16 ? mE : mF;
-        m[i * LM + j] = x;
-      }
-    }
-  }
-  __syncthreads();
-  if (tid < DC) {                              // column tid of (I + B)^-1, by forward substitution
-    float t[DC];
-#pragma unroll
-    for (int i = 0; i < DC; ++i) {
-      float s = 0.f;
-#pragma unroll
-      for (int l = 0; l < i; ++l) s = fmaf(mB[i * LM + l], t[l], s);
-      t[i] = (i == tid ? 1.f : 0.f) - s;
-      mT[i * LM + tid] = t[i];
-    }
-  }
-  __syncthreads();
-  float *mats = rec + 4 * DC * D + D;
-  for (int e = tid; e < DC * DC; e += DC_THREADS) {
-    const int i = (e >> 2) & 15, j = (e >> 6) * 4 + (e & 3);
-    float m = 0.f;
-    for (int l = 0; l <= i; ++l) m = fmaf(mT[i * LM + l], mA[l * LM + j], m);
-    mats[e] = mT[i * LM + j];
-    mats[DC * DC + e] = m;
-    mats[2 * DC * DC + e] = mE[i * LM + j];
-    mats[3 * DC * DC + e] = mF[i * LM + j];
-  }
-}
-
-__device__ __forceinline__ void fma_pair(unsigned long long &acc, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long both(float x) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float add_pair(unsigned long long x) { return __uint_as_float((unsigned)x) + __uint_as_float((unsigned)(x >> 32)); }
-
-// A CTA takes 32 columns of a head's state through a sequence's runs: four columns to 16 lanes, lane l rows 4 l .. 4 l + 3 of every 64.
-// What bounds it is the bytes from shared memory to registers (with a column to 8 lanes, each 16 bytes of a vector
-// met 4 multiplications and a run took 3.5 us; here they meet 16), so a vector's piece serves four columns, and the run's values and
-// removals stay in registers.  Records come through a ring of asynchronous copies; the only barrier is the ring's, one to a run.
-constexpr int DC_COLS = 32;
-template <int D>
-__global__ void __launch_bounds__(DC_THREADS)
-delta_chunk_scan_kernel(const float *__restrict__ proj, long long ld, int off_v, const float *__restrict__ records, float *__restrict__ state,
-                        float *__restrict__ out, long long ldo, const int *__restrict__ seq_start, const int *__restrict__ seq_slot,
-                        int n_heads, int d, int dv) {
-  constexpr int REC = delta_record(D), SLOT = REC + DC * DC_COLS, STAGES = D <= 64 ? 3 : 2, M = D / 64;
-  extern __shared__ __align__(16) float ring[];            // [STAGES][SLOT], then the column groups' rows [2][8][16][4]
-  float4 *xg = reinterpret_cast<float4 *>(ring + STAGES * SLOT), *xu = xg + 8 * DC;
-  const int b = blockIdx.x, hd = blockIdx.y, j0 = blockIdx.z * DC_COLS, tid = threadIdx.x;
-  const int sub = tid & 15, group = tid >> 4, j = j0 + 4 * group;            // this lane's columns: j .. j + 3
-  grid_dependency_wait();
-  int first = 0;
-  for (int s = 0; s < b; ++s) first += (seq_start[s + 1] - seq_start[s] + DC - 1) / DC;
-  const int start = seq_start[b], n = seq_start[b + 1] - start, runs = (n + DC - 1) / DC;
-  auto fetch = [&](int p) {
-    if (p < runs) {
-      float *dst = ring + (size_t)(p % STAGES) * SLOT;
-      const float *src = records + ((size_t)(first + p) * n_heads + hd) * REC;
-      for (int e = tid; e < REC / 4; e += DC_THREADS) cp_async16_cg(dst + 4 * e, src + 4 * e);
-#pragma unroll
-      for (int e = tid; e < DC * DC_COLS; e += DC_THREADS) {
-        const int t = p * DC + e / DC_COLS, c = j0 + e % DC_COLS;
-        if (t < n && c < dv) cp_async4(dst + REC + e, proj + (size_t)(start + t) * ld + off_v + (size_t)hd * dv + c);
-        else dst[REC + e] = 0.f;
-      }
-    }
-    cp_async_commit_group();
-  };
-  unsigned long long S[M][2][4];                           // rows 64 m + 4 sub + {0, 1}, {2, 3} of column c
-  float *sp = state + ((size_t)seq_slot[b] * n_heads + hd) * dv * d;
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int row = 64 * m + 4 * sub;
-      const ulonglong2 x = j + c < dv && row < d ? *reinterpret_cast<const ulonglong2 *>(sp + (size_t)(j + c) * d + row) : make_ulonglong2(0, 0);
-      S[m][0][c] = x.x;
-      S[m][1][c] = x.y;
-    }
-  // vectors at `vec` times the state, for the four columns: summed over the lanes, lane l keeps vector l's
-  auto times_state = [&](const float *vec, float (&y)[4]) {
-    float a[8][4];
-    const bool b3 = sub & 8, b2 = sub & 4, b1 = sub & 2, b0 = sub & 1;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      unsigned long long lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(vec + i * D + 64 * m + 4 * sub);
-        const ulonglong2 z = *reinterpret_cast<const ulonglong2 *>(vec + (i + 8) * D + 64 * m + 4 * sub);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          fma_pair(lo[c], x.x, S[m][0][c]);
-          fma_pair(hi[c], z.x, S[m][0][c]);
-          fma_pair(lo[c], x.y, S[m][1][c]);
-          fma_pair(hi[c], z.y, S[m][1][c]);
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float l = add_pair(lo[c]), h = add_pair(hi[c]);
-        a[i][c] = (b3 ? h : l) + __shfl_xor_sync(0xffffffffu, b3 ? l : h, 8);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float e[4], f[2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) e[i] = (b2 ? a[i + 4][c] : a[i][c]) + __shfl_xor_sync(0xffffffffu, b2 ? a[i][c] : a[i + 4][c], 4);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) f[i] = (b1 ? e[i + 2] : e[i]) + __shfl_xor_sync(0xffffffffu, b1 ? e[i] : e[i + 2], 2);
-      y[c] = (b0 ? f[1] : f[0]) + __shfl_xor_sync(0xffffffffu, b0 ? f[0] : f[1], 1);
-    }
-  };
-  // y += row `sub` of a matrix of the record times the sixteen rows r of four columns
-  auto times_rows = [&](const float *mat, const float4 (&r)[DC], float sign, float (&y)[4]) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 t = *reinterpret_cast<const float4 *>(mat + q * 64 + sub * 4);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float f = sign * (u == 0 ? t.x : u == 1 ? t.y : u == 2 ? t.z : t.w);
-        const float4 x = r[4 * q + u];
-        y[0] = fmaf(f, x.x, y[0]);
-        y[1] = fmaf(f, x.y, y[1]);
-        y[2] = fmaf(f, x.z, y[2]);
-        y[3] = fmaf(f, x.w, y[3]);
-      }
-    }
-  };
-  const bool quads = dv % 4 == 0 && ldo % 4 == 0 && (uintptr_t)out % 16 == 0;
-  for (int p = 0; p < STAGES - 1; ++p) fetch(p);
-  for (int p = 0; p < runs; ++p) {
-    cp_async_wait_group<STAGES - 2>();
-    __syncthreads();                                       // the run's record is there; everyone is done with the one before
-    fetch(p + STAGES - 1);
-    const float *rec = ring + (size_t)(p % STAGES) * SLOT, *mats = rec + 4 * DC * D + D;
-    float g[4], o[4], x[4] = {0.f, 0.f, 0.f, 0.f};
-    times_state(rec, g);
-    xg[group * DC + sub] = make_float4(g[0], g[1], g[2], g[3]);
-    times_state(rec + DC * D, o);
-    float4 v[DC], r[DC];
-#pragma unroll
-    for (int i = 0; i < DC; ++i) v[i] = *reinterpret_cast<const float4 *>(rec + REC + i * DC_COLS + 4 * group);
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < DC; ++i) r[i] = xg[group * DC + i];
-    times_rows(mats, r, 1.f, x);
-    times_rows(mats + DC * DC, v, 1.f, x);
-    xu[group * DC + sub] = make_float4(x[0], x[1], x[2], x[3]);
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < DC; ++i) r[i] = xu[group * DC + i];
-    times_rows(mats + 2 * DC * DC, v, 1.f, o);
-    times_rows(mats + 3 * DC * DC, r, -1.f, o);
-    const int t = p * DC + sub;
-    if (t < n) {
-      float *dst = out + (size_t)(start + t) * ldo + (size_t)hd * dv + j;
-      if (quads && j < dv) *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
-      else
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (j + c < dv) dst[c] = o[c];
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(rec + 4 * DC * D + 64 * m + 4 * sub);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        unsigned long long a = 0ull, e = 0ull;
-        fma_pair(a, w.x, S[m][0][c]);
-        fma_pair(e, w.y, S[m][1][c]);
-        S[m][0][c] = a;
-        S[m][1][c] = e;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < DC; ++i) {
-      const unsigned long long vi[4] = {both(v[i].x), both(v[i].y), both(v[i].z), both(v[i].w)};
-      const unsigned long long xi[4] = {both(-r[i].x), both(-r[i].y), both(-r[i].z), both(-r[i].w)};
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const ulonglong2 k = *reinterpret_cast<const ulonglong2 *>(rec + (2 * DC + i) * D + 64 * m + 4 * sub);
-        const ulonglong2 bb = *reinterpret_cast<const ulonglong2 *>(rec + (3 * DC + i) * D + 64 * m + 4 * sub);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          fma_pair(S[m][0][c], k.x, vi[c]);
-          fma_pair(S[m][1][c], k.y, vi[c]);
-          fma_pair(S[m][0][c], bb.x, xi[c]);
-          fma_pair(S[m][1][c], bb.y, xi[c]);
-        }
-      }
-    }
-  }
-  cp_async_wait_group<0>();
-  grid_dependents_launch();
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int row = 64 * m + 4 * sub;
-      if (j + c < dv && row < d) *reinterpret_cast<ulonglong2 *>(sp + (size_t)(j + c) * d + row) = make_ulonglong2(S[m][0][c], S[m][1][c]);
-    }
-}
-
-// Floats of scratch with which the recurrence takes sixteen tokens at a time, or 0 where it goes token by token: fewer than 32 tokens to a
-// sequence (a run of 16 costs as much as some eight tokens one by one), heads wider than 128 or not of whole pieces of four channels,
-// or more scratch than 1 GB.
-LLM_EXPORT long long llm_delta_chunk_floats(int n_tokens, int n_seqs, int n_heads, int d) {
-  if (n_tokens < 32 * n_seqs || d > 128 || d % 4 != 0) return 0;
-  const long long floats = ((long long)n_tokens / DC + n_seqs) * n_heads * delta_record(d <= 64 ? 64 : 128);
-  return floats <= (1ll << 28) ? floats : 0;
-}
-
-template <int D>
-static int launch_delta_chunks(const float *proj, long long ld, int off_r, int off_k, int off_v, const float *prep, float *records, float *state,
-                               float *out, long long ldo, const int *seq_start, const int *seq_slot, int n_tokens, int n_seqs, int n_heads,
-                               int d, int dv, cudaStream_t stream) {
-  const size_t smem = (size_t)(5 * DC * D + 5 * DC * (DC + 1)) * sizeof(float);
-  const size_t scan = (size_t)((D <= 64 ? 3 : 2) * (delta_record(D) + DC * DC_COLS) + 2 * 8 * DC * 4) * sizeof(float);
-  LLM_CHECK_CUDA(llm_allow_smem(delta_chunks_kernel<D>, smem), "delta_chunks attribute");
-  LLM_CHECK_CUDA(llm_allow_smem(delta_chunk_scan_kernel<D>, scan), "delta_chunk_scan attribute");
-  LLM_CHECK_CUDA(llm_launch(delta_chunks_kernel<D>, dim3(n_tokens / DC + n_seqs, n_heads), dim3(DC_THREADS), smem, stream, proj, ld, off_r, off_k,
-                            prep, seq_start, n_seqs, n_heads, d, records),
-                 "delta_chunks");
-  // behind its predecessor, like the token-by-token kernel: narrow and long
-  LLM_CHECK_CUDA(llm_launch_after(delta_chunk_scan_kernel<D>, dim3(n_seqs, n_heads, (dv + DC_COLS - 1) / DC_COLS), dim3(DC_THREADS), scan, stream, proj, ld,
-                                  off_v, (const float *)records, state, out, ldo, seq_start, seq_slot, n_heads, d, dv),
-                 "delta_chunk_scan");
-  return LLM_OK;
-}
-
-// The recurrence of prompts: token by token without scratch, or sixteen at a time with llm_delta_chunk_floats(..) floats of it.
-static int launch_delta(const float *proj, long long ld, int off_r, int off_k, int off_v, const float *prep, float *state, float *out, long long ldo,
-                        const int *seq_start, const int *seq_slot, int n_tokens, int n_seqs, int n_heads, int d, int dv, float *records,
-                        cudaStream_t stream) {
-  if (!records || (uintptr_t)state % 16 != 0 || (uintptr_t)records % 16 != 0)
-    return launch_delta_scan(proj, ld, off_r, off_k, off_v, prep, state, out, ldo, seq_start, seq_slot, n_seqs, n_heads, d, dv, stream);
-  LLM_REQUIRE(llm_delta_chunk_floats(n_tokens, n_seqs, n_heads, d) > 0, "delta_rule: no scratch is taken at these sizes");
-  return d <= 64 ? launch_delta_chunks<64>(proj, ld, off_r, off_k, off_v, prep, records, state, out, ldo, seq_start, seq_slot, n_tokens, n_seqs,
-                                           n_heads, d, dv, stream)
-                 : launch_delta_chunks<128>(proj, ld, off_r, off_k, off_v, prep, records, state, out, ldo, seq_start, seq_slot, n_tokens, n_seqs,
-                                            n_heads, d, dv, stream);
-}
-
-// `records`: scratch of llm_delta_chunk_floats floats (null, and where that is 0: the recurrence goes token by token).
 LLM_EXPORT int llm_delta_rule(const float *proj, long long ld, int off_r, int off_k, int off_v, int off_a, int off_x1, int rank,
                               const float *w2, const float *w0, const float *a_bias, float decay_scale, float key_eps,
                               float *prep, float *state, float *out, long long ldo, const int *seq_start, const int *seq_slot,
-                              int n_tokens, int n_seqs, int n_heads, int d, float *records, cudaStream_t stream) {
+                              int n_tokens, int n_seqs, int n_heads, int d, cudaStream_t stream) {
   if (n_tokens == 0) return LLM_OK;
   LLM_REQUIRE(n_tokens > 0 && n_seqs > 0 && n_heads > 0 && d > 0 && rank > 0, "delta_rule: bad sizes");
   LLM_REQUIRE(d <= 256, "delta_rule: heads of %d channels are not supported (up to 256)", d);
@@ -892,19 +520,19 @@ LLM_EXPORT int llm_delta_rule(const float *proj, long long ld, int off_r, int of
                proj, ld, off_k, off_a, off_x1, rank, w2, w0, a_bias, decay_scale, key_eps, n_tokens, n_heads, d, w2_shared, prep);
     LLM_CHECK_LAUNCH("delta_prepare");
   }
-  return launch_delta(proj, ld, off_r, off_k, off_v, prep, state, out, ldo, seq_start, seq_slot, n_tokens, n_seqs, n_heads, d, d, records, stream);
+  return launch_delta_scan(proj, ld, off_r, off_k, off_v, prep, state, out, ldo, seq_start, seq_slot, n_seqs, n_heads, d, d, stream);
 }
 
 // The recurrence alone, for a mixer that prepares the tokens' vectors itself: rows `proj` (32-bit) hold r and k
-// (heads x d each) and v (heads x dv), `prep` [tokens, heads, 3, d] holds w, b, u; state [slots, heads, dv, d]; records as above.
+// (heads x d each) and v (heads x dv), `prep` [tokens, heads, 3, d] holds w, b, u; state [slots, heads, dv, d].
 LLM_EXPORT int llm_delta_scan(const float *proj, long long ld, int off_r, int off_k, int off_v, const float *prep, float *state,
                               float *out, long long ldo, const int *seq_start, const int *seq_slot, int n_tokens, int n_seqs,
-                              int n_heads, int d, int dv, float *records, cudaStream_t stream) {
+                              int n_heads, int d, int dv, cudaStream_t stream) {
   if (n_tokens == 0) return LLM_OK;
   LLM_REQUIRE(n_tokens > 0 && n_seqs > 0 && n_heads > 0 && d > 0 && dv > 0, "delta_scan: bad sizes");
   LLM_REQUIRE(d <= 256, "delta_scan: heads of %d key channels are not supported (up to 256)", d);
   LLM_REQUIRE(n_heads <= 65535 && n_seqs < 2147483647, "delta_scan: too many heads or sequences");
-  return launch_delta(proj, ld, off_r, off_k, off_v, prep, state, out, ldo, seq_start, seq_slot, n_tokens, n_seqs, n_heads, d, dv, records, stream);
+  return launch_delta_scan(proj, ld, off_r, off_k, off_v, prep, state, out, ldo, seq_start, seq_slot, n_seqs, n_heads, d, dv, stream);
 }
 
 // ---------------------------------------------------------------- the delta rule: a step of single tokens

@@ -100,11 +100,9 @@ class GeneralDelta : public Mixer {
       return linear(ctx, y, w_o_, nullptr, DType::F32, true);
     }
     float *prep = ctx.arena->alloc_n<float>((size_t)T * (size_t)width_ * 3);
-    const size_t scratch = kernels::delta_chunk_floats(T, ctx.n_seqs, n_heads_, d_);
-    float *records = scratch ? ctx.arena->alloc_n<float>(scratch) : nullptr;
     Act o = ctx.arena->act(DType::F32, T, width_);
     kernels::delta_rule(proj, 0, W, 2 * W, 4 * W, 5 * W, (int)rank_, w2_.buf.as<float>(), w0_.buf.as<float>(), a_bias_.buf.as<float>(),
-                        decay_scale_, key_eps_, prep, S, o, ctx.seq_start, ctx.seq_slot, ctx.n_seqs, n_heads_, d_, records, ctx.stream);
+                        decay_scale_, key_eps_, prep, S, o, ctx.seq_start, ctx.seq_slot, ctx.n_seqs, n_heads_, d_, ctx.stream);
     Act y = ctx.arena->act(ctx.dtype, T, width_);
     kernels::head_norm_gate(o, norm_.buf.as<float>(), (const float *)proj.data + 3 * W, proj.ld, eps_, n_heads_, d_, y, ctx.stream);
     return linear(ctx, y, w_o_, nullptr, DType::F32, true);
@@ -254,11 +252,9 @@ class ChannelDelta : public Mixer {
     kernels::channel_delta_prepare(cv, proj, (int)off_b_, (int)off_a1_, (int)rank_a_, (int)off_g1_, (int)rank_g_, a2_.buf.as<float>(),
                                    dt_bias_.buf.as<float>(), a_log_.buf.as<float>(), g2_.buf.as<float>(), key_eps_, prep, gate, n_heads_,
                                    n_kv_, d_, dv_, ctx.stream);
-    const size_t scratch = kernels::delta_chunk_floats(T, ctx.n_seqs, n_heads_, d_);
-    float *records = scratch ? ctx.arena->alloc_n<float>(scratch) : nullptr;
     Act o = ctx.arena->act(DType::F32, T, v_width_);
     kernels::delta_scan(cv, (int)conv_width_, (int)(conv_width_ + k_width_), (int)(2 * qk_width_), prep, S, o, ctx.seq_start, ctx.seq_slot,
-                        ctx.n_seqs, n_heads_, d_, dv_, records, ctx.stream);
+                        ctx.n_seqs, n_heads_, d_, dv_, ctx.stream);
     Act y = ctx.arena->act(ctx.dtype, T, v_width_);
     kernels::head_norm_gate(o, norm_.buf.as<float>(), gate, v_width_, eps_, n_heads_, dv_, y, ctx.stream);
     return linear(ctx, y, w_o_, nullptr, DType::F32, true);

@@ -132,6 +132,27 @@ def test_first_tokens_beside_a_long_neighbour(dtype):
     compare(both["l"], "S1", c, w, long_, dtype, "long neighbour")
 
 
+def test_logits_are_the_same_in_any_company():
+    """A prompt's 32-bit logits, and those of the tokens behind it, to the bit: alone, beside single-token sequences, and in portions."""
+    engine, c, w = setup("S6", "float32")
+    toks = S.tokens(c, 50, 8)
+
+    def request(neighbours, portions):
+        slots = [engine.open_sequence() for _ in range(neighbours + 1)]
+        rows, at = [], 0
+        for n in portions + [2] * ((50 - sum(portions)) // 2):      # two tokens at a time: the prompt's form of every kernel
+            got = engine.step([StepItem(slots[0], toks[at:at + n], list(range(n)))] + [StepItem(s, [5], [0]) for s in slots[1:]])
+            rows.append(torch.from_numpy(got)[:n])
+            at += n
+        for s in slots:
+            engine.close_sequence(s)
+        return torch.cat(rows)
+
+    alone = request(0, [40])
+    assert torch.equal(request(3, [40]), alone)
+    assert torch.equal(request(1, [19, 21]), alone)
+
+
 @pytest.mark.parametrize("name", NAMES)
 def test_pages_outside_the_window_come_back_but_the_first_ones_stay(name):
     """A window's group holds the pages of the window and of the kept first tokens, no more."""
