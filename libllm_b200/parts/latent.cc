@@ -211,15 +211,12 @@ class LatentAttention : public Mixer {
     Act mixed = ctx.arena->act(ctx.dtype, T, (int64_t)n_heads_ * kv_rank_);
     if (tc && kernels::latent_decode_supported(kv_rank_, rot_)) {
       // all heads of a token over the cached rows.  A run's partial result is heads x kv_rank 32-bit sums, as many
-      // bytes as some tens of cached rows, so a run takes at least 256 keys (128 under a window, where a token has few);
-      // within that, enough runs to give every multiprocessor a CTA.  Where runs of 256 leave multiprocessors without one, a tile of 64 is run
-      // enough: two sequences of 2,000 positions had 16 CTAs that walked four tiles in 28 us, 64 CTAs take 12 and the join
-      // 6.6 (runs of 128: 18 and 4.6).  The same for every step of a captured graph.
+      // bytes as some tens of cached rows, so a run takes at least 256 keys; within that, enough runs to give
+      // every multiprocessor a CTA.  The same for every step of a captured graph.
       const int max_len = window_ > 0 ? std::min(std::max(ctx.max_kv_len, 1), window_ + 63) : std::max(ctx.max_kv_len, 1);
       const int ctas = std::max(1, T * ((n_heads_ + 31) / 32));
       const int want = std::max(1, (ctx.sm_count + ctas - 1) / ctas);
-      const int run = ctas * (max_len / 256) < ctx.sm_count ? 64 : window_ > 0 ? 128 : 256;
-      const int most = std::max(1, max_len / run);
+      const int most = std::max(1, max_len / (window_ > 0 ? 128 : 256));      // under a window a token has few keys: shorter runs, more CTAs
       const int n_splits = std::max(1, std::min(std::min(want, most), 64));
       float *ws = nullptr;
       if (n_splits > 1) ws = ctx.arena->alloc_n<float>(kernels::latent_decode_floats(T, n_heads_, kv_rank_, n_splits));

@@ -208,6 +208,20 @@ def test_latent_prompt_and_token_by_token_are_one_function(sizes):
             close(other[i][0], results[0][i][0].double(), "bfloat16", f"latent layer {i} in single tokens", roundings=4.0)
 
 
+def test_latent_tokens_behind_cached_rows_are_the_same_alone_and_together():
+    """Eighty tokens behind 220 cached ones, at once and one at a time: below 512 positions a token's keys are one run whatever else
+    the step holds, so the results are the same bits."""
+    layers, built = latent_pair(LATENT_SIZES[1], "bfloat16", 13)
+    x = sharp_inputs(7, [300])
+    row = LATENT_SIZES[1][4] + LATENT_SIZES[1][2]
+    results = []
+    for portions in ([[220], [80]], [[220]] + [[1]] * 80):
+        k = torch.zeros(N_PAGES, PAGE, row, dtype=torch.bfloat16, device=DEV)
+        results.append(run_in_portions([b[0] for b in built], [(k, None, True), (k, None, False)], x, portions, "bfloat16", [300]))
+    for i in range(2):
+        assert torch.equal(results[0][i][0], results[1][i][0]), f"latent layer {i}"
+
+
 # tokens at which another instantiation takes over, heads of one and of several fetches of w_uk, latents with an odd width
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,H,d,rot,R,dv", [(1, 2, 6, 2, 22, 10), (2, 3, 64, 32, 512, 64), (3, 1, 65, 0, 33, 7), (4, 2, 80, 4, 520, 9),
