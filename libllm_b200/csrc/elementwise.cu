@@ -173,6 +173,14 @@ LLM_EXPORT int llm_gather_words(const int *src1, int n1, const int *src2, int n2
 }
 
 // ---------------------------------------------------------------- add + rmsnorm
+// What a scaled addition rounds is fixed by name, for a compiler joins multiplication and addition in one kernel and not in
+// another, and a result would change with whatever else is changed here.  JOINED: one rounding, where several parts are added to
+// rows of up to 4,096 columns (a cut product's sums); everywhere else the product is rounded before it is added.
+template <bool JOINED>
+__device__ __forceinline__ float scaled_sum(float v, float d, float bias, float scale) {
+  return JOINED ? fmaf(d + bias, scale, v) : __fadd_rn(v, __fmul_rn(d + bias, scale));
+}
+
 // For each output row i (source row r = rows ? rows[i] : i):
 //   v = resid[r] + sum_p delta[p][r]      (32-bit; parts added in index order)
 //       with col_scale / col_bias (vectors over the columns, either may be null):
@@ -198,9 +206,7 @@ __global__ void add_rmsnorm_kernel(float *__restrict__ resid, const TD *__restri
     if (col_scale || col_bias) {
       float d = 0.f;
       for (int p = 0; p < n_parts; ++p) d += to_float(delta[p * part_stride + (size_t)r * hidden + c]);
-      if (col_bias) d += col_bias[c];
-      if (col_scale) d *= col_scale[c];
-      if (n_parts > 0) v += d;
+      if (n_parts > 0) v = scaled_sum<false>(v, d, col_bias ? col_bias[c] : 0.f, col_scale ? col_scale[c] : 1.f);
     } else {
       for (int p = 0; p < n_parts; ++p) v += to_float(delta[p * part_stride + (size_t)r * hidden + c]);
     }
@@ -276,10 +282,10 @@ add_rmsnorm_vec_kernel(float *__restrict__ resid, const TD *__restrict__ delta, 
             t.z += d[j][p].z;
             t.w += d[j][p].w;
           }
-        v[j].x = fmaf(t.x + cb[j].x, cs[j].x, v[j].x);
-        v[j].y = fmaf(t.y + cb[j].y, cs[j].y, v[j].y);
-        v[j].z = fmaf(t.z + cb[j].z, cs[j].z, v[j].z);
-        v[j].w = fmaf(t.w + cb[j].w, cs[j].w, v[j].w);
+        v[j].x = scaled_sum<VPT == 1 && (MAXP > 1)>(v[j].x, t.x, cb[j].x, cs[j].x);
+        v[j].y = scaled_sum<VPT == 1 && (MAXP > 1)>(v[j].y, t.y, cb[j].y, cs[j].y);
+        v[j].z = scaled_sum<VPT == 1 && (MAXP > 1)>(v[j].z, t.z, cb[j].z, cs[j].z);
+        v[j].w = scaled_sum<VPT == 1 && (MAXP > 1)>(v[j].w, t.w, cb[j].w, cs[j].w);
       } else {
 #pragma unroll
         for (int p = 0; p < MAXP; ++p)
@@ -337,13 +343,13 @@ norm_rows_kernel(float *__restrict__ resid, const TD *__restrict__ delta, const 
       const int c4 = lane + j * 32;
       if (c4 < n4) {
         const float4 t = ld4(d + 4 * c4);
-        if (col_scale || col_bias) {         // spelled out, here and above: a compiler may or may not join the two by itself
+        if (col_scale || col_bias) {
           const float4 cs = col_scale ? ld4(col_scale + 4 * c4) : make_float4(1.f, 1.f, 1.f, 1.f);
           const float4 cb = col_bias ? ld4(col_bias + 4 * c4) : make_float4(0.f, 0.f, 0.f, 0.f);
-          v[j].x = fmaf(t.x + cb.x, cs.x, v[j].x);
-          v[j].y = fmaf(t.y + cb.y, cs.y, v[j].y);
-          v[j].z = fmaf(t.z + cb.z, cs.z, v[j].z);
-          v[j].w = fmaf(t.w + cb.w, cs.w, v[j].w);
+          v[j].x = scaled_sum<false>(v[j].x, t.x, cb.x, cs.x);
+          v[j].y = scaled_sum<false>(v[j].y, t.y, cb.y, cs.y);
+          v[j].z = scaled_sum<false>(v[j].z, t.z, cb.z, cs.z);
+          v[j].w = scaled_sum<false>(v[j].w, t.w, cb.w, cs.w);
         } else {
           v[j].x += t.x;
           v[j].y += t.y;

@@ -487,6 +487,33 @@ def test_tensor_core_product_in_parts_of_k(M, N, K, parts):
     assert 1 <= ops.gemm_tc_suggest_parts(M, N, K) <= 8
 
 
+# one part, several and more than the registers for eight; a width for a block of each size, one for four pieces to a thread and one
+# without 16-byte rows; few rows and prompt rows
+@pytest.mark.parametrize("hidden", [1000, 1030, 2048, 4096, 4100])
+@pytest.mark.parametrize("parts", [1, 2, 6, 12])
+def test_what_a_scaled_addition_rounds(hidden, parts):
+    """resid + (sum + bias) * scale to the bit: the product rounded, then the sum; both at once for several parts of rows of up to 4,096."""
+    from ctypes import c_float, c_int, c_longlong, c_void_p
+    from libllm_b200.csrc import ops
+    P_, I_ = c_void_p, c_int
+    for rows in (5, 1030):
+        g = torch.Generator().manual_seed(hidden + parts)
+        x, d = torch.randn(rows, hidden, generator=g), torch.randn(parts, rows, hidden, generator=g)
+        s, b, w = (torch.randn(hidden, generator=g) for _ in range(3))
+        t = d[0].clone()
+        for p in range(1, parts):
+            t = t + d[p]
+        t = t + b
+        joined = parts > 1 and hidden % 4 == 0 and hidden <= 4096
+        want = (x.double() + t.double() * s.double()).float() if joined else x + t * s      # 48 bits of a product are exact in 64
+        X, D, S, B, W = (v.to(DEV) for v in (x, d, s, b, w))
+        out = torch.empty_like(X)
+        ops._call("elementwise", "llm_add_rmsnorm_scaled", [P_, P_, I_, I_, c_longlong, P_, c_float, P_, I_, P_, I_, I_, P_, P_, P_],
+                  X.data_ptr(), D.data_ptr(), 0, parts, rows * hidden, W.data_ptr(), 1e-5, out.data_ptr(), 0, None, rows, hidden,
+                  S.data_ptr(), B.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(X.cpu(), want)
+
+
 # widths at and beside a lane's pieces, the row count at which the prompt kernel takes over and one that leaves a CTA's last warps idle
 @pytest.mark.parametrize("hidden", [516, 1024, 1028, 2048, 2052, 3072, 4092, 4096])
 @pytest.mark.parametrize("parts,scaled", [(0, False), (1, False), (1, True)])
