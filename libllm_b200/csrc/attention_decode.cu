@@ -34,12 +34,12 @@ __device__ __forceinline__ void unpack8(const uint4 &raw, float (&f)[8]) {
 
 template <int D, int G>
 __global__ void __launch_bounds__(AD_THREADS)
-attention_decode_kernel(const __nv_bfloat16 *__restrict__ q, long long q_stride,
-                        const __nv_bfloat16 *__restrict__ kc, const __nv_bfloat16 *__restrict__ vc,
-                        const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride,
+attention_decode_kernel(const __nv_bfloat16 *q, long long q_stride,
+                        const __nv_bfloat16 *kc, const __nv_bfloat16 *vc,
+                        const int *tok_pos, const int *page_table, int pt_stride,
                         int n_kv, int page_size, int chunk, int window, int block, int sink, float scale_log2,
                         float *__restrict__ ws_o, float *__restrict__ ws_ml, int n_splits,
-                        __nv_bfloat16 *__restrict__ out, long long out_stride, const float *__restrict__ gate,
+                        __nv_bfloat16 *__restrict__ out, long long out_stride, const float *gate,
                         long long gate_stride, int gate_per_channel, float null_log2, const float *__restrict__ null_scores) {
   constexpr int LPK = D / 8;                 // lanes per key
   constexpr int GPW = 32 / LPK;              // lane groups per warp
@@ -234,10 +234,10 @@ attention_decode_kernel(const __nv_bfloat16 *__restrict__ q, long long q_stride,
 }
 
 // Joins the splits of one (sequence, head): out = sum_s o_s 2^(m_s - M) / sum_s l_s 2^(m_s - M).
-__global__ void attention_decode_combine_kernel(const float *__restrict__ ws_o, const float *__restrict__ ws_ml,
-                                                const int *__restrict__ tok_pos, int n_heads, int D, int chunk,
+__global__ void attention_decode_combine_kernel(const float *ws_o, const float *ws_ml,
+                                                const int *tok_pos, int n_heads, int D, int chunk,
                                                 int window, int block, int sink, int n_splits, __nv_bfloat16 *__restrict__ out,
-                                                long long out_stride, const float *__restrict__ gate,
+                                                long long out_stride, const float *gate,
                                                 long long gate_stride, int gate_per_channel, float null_log2,
                                                 const float *__restrict__ null_scores) {
   grid_dependents_launch();

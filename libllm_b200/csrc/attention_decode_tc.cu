@@ -60,14 +60,14 @@ __host__ __device__ constexpr int decode_tc_ctas(int dmax) { return dmax <= 64 ?
 
 template <int D, int DV, bool EXACT, int DT_WARPS>
 __global__ void __launch_bounds__(DT_WARPS * 32, decode_tc_ctas(D > DV ? D : DV))
-attention_decode_tc_kernel(const float *__restrict__ qkv, long long qkv_stride, int qkv_parts,
+attention_decode_tc_kernel(const float *qkv, long long qkv_stride, int qkv_parts,
                            long long qkv_part_stride, const float *__restrict__ table,
-                           int table_rows, int rot_dim, const int *__restrict__ tok_pos,
-                           const int *__restrict__ page_table, int pt_stride, __nv_bfloat16 *__restrict__ kc,
-                           __nv_bfloat16 *__restrict__ vc, int write_cache, int n_heads, int n_kv, int G, int d_arg, int dv_arg,
+                           int table_rows, int rot_dim, const int *tok_pos,
+                           const int *page_table, int pt_stride, __nv_bfloat16 *kc,
+                           __nv_bfloat16 *vc, int write_cache, int n_heads, int n_kv, int G, int d_arg, int dv_arg,
                            int chunk, int window, int block, float scale_log2, const float *__restrict__ bias,
-                           const float *__restrict__ null_scores, float *__restrict__ ws_o, float *__restrict__ ws_ml,
-                           int *__restrict__ counters, int n_splits, __nv_bfloat16 *__restrict__ out,
+                           const float *__restrict__ null_scores, float *ws_o, float *ws_ml,
+                           int *counters, int n_splits, __nv_bfloat16 *__restrict__ out,
                            long long out_stride) {
   const int d = EXACT ? D : d_arg, dv = EXACT ? DV : dv_arg;
   constexpr int LD = D + 8, LDV = DV + 8;

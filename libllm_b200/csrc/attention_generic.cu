@@ -77,12 +77,12 @@ struct SigmoidWeights {
 
 template <typename T, int MAX_D, bool SIG>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_generic_kernel(const T *__restrict__ q, long long q_stride, T *__restrict__ out,
-                         long long out_stride, const T *__restrict__ kcache,
-                         const T *__restrict__ vcache, const int *__restrict__ tok_seq,
-                         const int *__restrict__ tok_pos, const int *__restrict__ page_table,
+attention_generic_kernel(const T *q, long long q_stride, T *__restrict__ out,
+                         long long out_stride, const T *kcache,
+                         const T *vcache, const int *tok_seq,
+                         const int *tok_pos, const int *page_table,
                          int pt_stride, int n_heads, int n_kv, int d, int dv, int page_size,
-                         int window, int block, int sink, float scale, const float *__restrict__ gate,
+                         int window, int block, int sink, float scale, const float *gate,
                          long long gate_stride, int vec, int v_ld, float null_score, const float *__restrict__ null_scores,
                          SigmoidWeights sig) {
   __shared__ __align__(16) float q_s[MAX_D];

@@ -33,10 +33,10 @@ constexpr int AP_BN = 64;                // keys per tile = tokens per page
 
 template <int D>
 __global__ void __launch_bounds__(AP_WARPS * 32)
-attention_prefill_kernel(const __nv_bfloat16 *__restrict__ q, long long q_stride, __nv_bfloat16 *__restrict__ out,
-                         long long out_stride, const __nv_bfloat16 *__restrict__ kc,
-                         const __nv_bfloat16 *__restrict__ vc, const int *__restrict__ seq_start,
-                         const int *__restrict__ seq_past, const int *__restrict__ page_table, int pt_stride,
+attention_prefill_kernel(const __nv_bfloat16 *q, long long q_stride, __nv_bfloat16 *__restrict__ out,
+                         long long out_stride, const __nv_bfloat16 *kc,
+                         const __nv_bfloat16 *vc, const int *seq_start,
+                         const int *seq_past, const int *page_table, int pt_stride,
                          int n_heads, int n_kv, int window, int block, int sink, float scale_log2, float null_log2,
                          const float *__restrict__ null_scores) {
   constexpr int LD = D + 8;                                  // padded row, in elements

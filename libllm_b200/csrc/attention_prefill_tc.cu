@@ -90,8 +90,8 @@ template <int KB, int VB>
 __global__ void __launch_bounds__(FT_THREADS, FtShape<KB, VB>::CTAS)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, __nv_bfloat16 *__restrict__ out,
-                            long long out_stride, const int *__restrict__ seq_start, const int *__restrict__ seq_past,
-                            const int *__restrict__ page_table, int pt_stride, int n_heads, int n_kv, int d, int dv, int window,
+                            long long out_stride, const int *seq_start, const int *seq_past,
+                            const int *page_table, int pt_stride, int n_heads, int n_kv, int d, int dv, int window,
                             int block, int sink, float scale_log2, float null_log2, const float *__restrict__ null_scores,
                             int *status) {
   using S = FtShape<KB, VB>;
@@ -471,8 +471,8 @@ template <int D>
 __global__ void __launch_bounds__(FW_THREADS, 1)
 attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                               const __grid_constant__ CUtensorMap map_v, __nv_bfloat16 *__restrict__ out,
-                              long long out_stride, const int *__restrict__ seq_start, const int *__restrict__ seq_past,
-                              const int *__restrict__ page_table, int pt_stride, int n_heads, int n_kv, int window, int block,
+                              long long out_stride, const int *seq_start, const int *seq_past,
+                              const int *page_table, int pt_stride, int n_heads, int n_kv, int window, int block,
                               float scale_log2, float null_log2, const float *__restrict__ null_scores, int *status) {
   using S = FwShape<D>;
   constexpr int STAGES = S::STAGES;

@@ -98,7 +98,7 @@ template <int KB, int VB, bool BOUNDED>
 __global__ void __launch_bounds__(SA_THREADS, SaShape<KB, VB>::CTAS)
 sigmoid_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, __nv_bfloat16 *__restrict__ out, long long out_stride,
-                       const int *__restrict__ seq_start, const int *__restrict__ seq_past, const int *__restrict__ page_table,
+                       const int *seq_start, const int *seq_past, const int *page_table,
                        int pt_stride, int n_heads, int n_kv, int d, int dv, int window, float scale, const float *__restrict__ temp,
                        const float *__restrict__ bias, float cap, float out_scale, int *status) {
   using S = SaShape<KB, VB>;
@@ -395,11 +395,11 @@ constexpr int SD_WARPS = 4, SD_BN = 64;
 
 template <int VT>                           // 16-channel groups of the value a warp owns at most
 __global__ void __launch_bounds__(SD_WARPS * 32)
-sigmoid_decode_kernel(const __nv_bfloat16 *__restrict__ q, long long q_stride, const __nv_bfloat16 *__restrict__ kc,
-                      const __nv_bfloat16 *__restrict__ vc, const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride,
+sigmoid_decode_kernel(const __nv_bfloat16 *q, long long q_stride, const __nv_bfloat16 *kc,
+                      const __nv_bfloat16 *vc, const int *tok_pos, const int *page_table, int pt_stride,
                       int n_heads, int n_kv, int d, int dv, int window, float scale, const float *__restrict__ temp,
-                      const float *__restrict__ bias, float cap, float out_scale, int n_splits, float *__restrict__ ws,
-                      int *__restrict__ counters, __nv_bfloat16 *__restrict__ out, long long out_stride) {
+                      const float *__restrict__ bias, float cap, float out_scale, int n_splits, float *ws,
+                      int *counters, __nv_bfloat16 *__restrict__ out, long long out_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ldk = d + 8, ldv = dv + 8;
   constexpr int LDP = SD_BN + 8;

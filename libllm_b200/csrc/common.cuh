@@ -63,6 +63,13 @@ static thread_local char g_llm_error[512] = "";
 // arithmetic, loads of weights) overlaps the predecessor's tail.  Every thread of every
 // kernel launched this way calls the wait, so completion stays transitive along the stream.
 // Without the launch attribute both calls do nothing.
+//
+// The wait orders a read behind it only if the compiler does.  `__restrict__` on a pointer says that nothing else in the kernel, the
+// wait included, touches what lies there, and `const T *__restrict__` that it does not change while the kernel lives: either lets a
+// load move in front of the wait, where the kernel before may still be storing.  So in a kernel that waits,
+//   * `const T *__restrict__` is for what no kernel of a step writes: weights, biases, tables;
+//   * `T *__restrict__` is for what the kernel only stores;
+//   * rows, caches, states, positions, page tables and scratch that it reads have plain pointers (also in the functions it calls).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -152,7 +159,7 @@ __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) {
 
 // Four consecutive values as 32-bit floats, from or to either element type.
 // the sum of the `parts` partial results p[0], p[stride], .., in that order, eight on their way at once
-__device__ __forceinline__ float sum_parts(const float *__restrict__ p, int parts, long long stride) {
+__device__ __forceinline__ float sum_parts(const float *p, int parts, long long stride) {
   if (parts == 1) return p[0];
   float sum = 0.f;
   for (int p0 = 0; p0 < parts; p0 += 8) {

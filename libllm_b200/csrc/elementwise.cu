@@ -24,10 +24,10 @@ struct TokenExtras {
 };
 
 template <typename T>
-__global__ void embedding_kernel(const T *__restrict__ table, const int *__restrict__ tokens,
-                                 const int *__restrict__ fed_tokens, const int *__restrict__ fed_rows,
+__global__ void embedding_kernel(const T *__restrict__ table, const int *tokens,
+                                 const int *fed_tokens, const int *fed_rows,
                                  float *__restrict__ out, int hidden, int vocab, const T *__restrict__ pos_table,
-                                 int pos_rows, const int *__restrict__ tok_pos, TokenExtras ex) {
+                                 int pos_rows, const int *tok_pos, TokenExtras ex) {
   grid_dependents_launch();
   grid_dependency_wait();
   const int t = blockIdx.x;
@@ -135,7 +135,7 @@ LLM_EXPORT int llm_embedding(int dtype, const void *table, const int *tokens, co
 // a kernel two or three.
 // The kernels behind it may start only when the words are written: later kernels of a step read
 // the descriptor before they wait for their predecessors.
-__global__ void copy_words_kernel(const int *__restrict__ src, int *__restrict__ dst, int n) {
+__global__ void copy_words_kernel(const int *src, int *__restrict__ dst, int n) {
   grid_dependency_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
   __threadfence();
@@ -153,7 +153,7 @@ LLM_EXPORT int llm_copy_words(const int *src, int *dst, int n, cudaStream_t stre
 
 // n1 words from src1 followed by n2 words from src2, to dst (which may be pinned host memory): a
 // step's sampled tokens and the status word of its tensor-core kernels leave the device together.
-__global__ void gather_words_kernel(const int *__restrict__ src1, int n1, const int *__restrict__ src2, int n2,
+__global__ void gather_words_kernel(const int *src1, int n1, const int *src2, int n2,
                                     int *__restrict__ dst) {
   grid_dependency_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n1 + n2; i += gridDim.x * blockDim.x)
@@ -188,9 +188,9 @@ __device__ __forceinline__ float scaled_sum(float v, float d, float bias, float 
 //   if (!rows) resid[r] = v               (the residual stream moves on)
 //   out[i] = v * w * rsqrt(mean(v^2) + eps)   (skipped when out is null)
 template <typename TD, typename TO, int THREADS>
-__global__ void add_rmsnorm_kernel(float *__restrict__ resid, const TD *__restrict__ delta,
+__global__ void add_rmsnorm_kernel(float *resid, const TD *delta,
                                    int n_parts, size_t part_stride, const float *__restrict__ weight,
-                                   float eps, TO *__restrict__ out, const int *__restrict__ rows,
+                                   float eps, TO *__restrict__ out, const int *rows,
                                    int hidden, const float *__restrict__ col_scale,
                                    const float *__restrict__ col_bias) {
   extern __shared__ float row_buf[];   // hidden floats
@@ -229,9 +229,9 @@ __global__ void add_rmsnorm_kernel(float *__restrict__ resid, const TD *__restri
 // result does not depend on the other rows of the launch.
 template <typename TD, typename TO, int THREADS, int VPT, int MAXP>
 __global__ void __launch_bounds__(THREADS)
-add_rmsnorm_vec_kernel(float *__restrict__ resid, const TD *__restrict__ delta, int n_parts,
+add_rmsnorm_vec_kernel(float *resid, const TD *delta, int n_parts,
                        size_t part_stride, const float *__restrict__ weight, float eps,
-                       TO *__restrict__ out, const int *__restrict__ rows, int hidden,
+                       TO *__restrict__ out, const int *rows, int hidden,
                        const float *__restrict__ col_scale, const float *__restrict__ col_bias) {
   __shared__ float scratch[THREADS / 32 + 1];
   grid_dependents_launch();
@@ -323,7 +323,7 @@ add_rmsnorm_vec_kernel(float *__restrict__ resid, const TD *__restrict__ delta, 
 // 2,048 rows of 2,048: 8.0 -> 5.1 us; 8,192 of 3,072: 39 -> 23; 8,192 of 4,096: 69 -> 44 (201 MB: 4.6 TB/s).
 template <typename TD, typename TO, int VPL, bool DELTA>
 __global__ void __launch_bounds__(128)
-norm_rows_kernel(float *__restrict__ resid, const TD *__restrict__ delta, const float *__restrict__ weight, float eps,
+norm_rows_kernel(float *resid, const TD *delta, const float *__restrict__ weight, float eps,
                  TO *__restrict__ out, int n_rows, int hidden, const float *__restrict__ col_scale, const float *__restrict__ col_bias) {
   grid_dependents_launch();
   const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5), n4 = hidden / 4;
@@ -338,23 +338,28 @@ norm_rows_kernel(float *__restrict__ resid, const TD *__restrict__ delta, const 
   }
   if (DELTA) {
     const TD *d = delta + (size_t)row * hidden;
+    float4 t[VPL];
+#pragma unroll
+    for (int j = 0; j < VPL; ++j) {
+      const int c4 = lane + j * 32;
+      t[j] = c4 < n4 ? ld4(d + 4 * c4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
       const int c4 = lane + j * 32;
       if (c4 < n4) {
-        const float4 t = ld4(d + 4 * c4);
         if (col_scale || col_bias) {
           const float4 cs = col_scale ? ld4(col_scale + 4 * c4) : make_float4(1.f, 1.f, 1.f, 1.f);
           const float4 cb = col_bias ? ld4(col_bias + 4 * c4) : make_float4(0.f, 0.f, 0.f, 0.f);
-          v[j].x = scaled_sum<false>(v[j].x, t.x, cb.x, cs.x);
-          v[j].y = scaled_sum<false>(v[j].y, t.y, cb.y, cs.y);
-          v[j].z = scaled_sum<false>(v[j].z, t.z, cb.z, cs.z);
-          v[j].w = scaled_sum<false>(v[j].w, t.w, cb.w, cs.w);
+          v[j].x = scaled_sum<false>(v[j].x, t[j].x, cb.x, cs.x);
+          v[j].y = scaled_sum<false>(v[j].y, t[j].y, cb.y, cs.y);
+          v[j].z = scaled_sum<false>(v[j].z, t[j].z, cb.z, cs.z);
+          v[j].w = scaled_sum<false>(v[j].w, t[j].w, cb.w, cs.w);
         } else {
-          v[j].x += t.x;
-          v[j].y += t.y;
-          v[j].z += t.z;
-          v[j].w += t.w;
+          v[j].x += t[j].x;
+          v[j].y += t[j].y;
+          v[j].z += t[j].z;
+          v[j].w += t[j].w;
         }
         st4(x + 4 * c4, v[j]);
       }
@@ -511,9 +516,9 @@ __device__ __forceinline__ void block_sums(float (&v)[N], float *scratch /* N * 
 // General form: rows of any width, two rows of `hidden` floats in shared memory.
 template <typename TO, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-stream_norm_kernel(float *__restrict__ resid, const float *__restrict__ delta, int n_parts, size_t part_stride,
+stream_norm_kernel(float *resid, const float *delta, int n_parts, size_t part_stride,
                    const float *__restrict__ col_bias, ResultNorms rn, const float *__restrict__ weight, float eps, TO *__restrict__ out,
-                   const int *__restrict__ rows, float *__restrict__ resid_out, int hidden) {
+                   const int *rows, float *__restrict__ resid_out, int hidden) {
   extern __shared__ float norm_rows[];
   float *ya = norm_rows, *yb = norm_rows + hidden;
   __shared__ float scratch[2 * (THREADS / 32 + 1)];
@@ -570,9 +575,9 @@ stream_norm_kernel(float *__restrict__ resid, const float *__restrict__ delta, i
 // weights) is issued before the first sum.  PAIR: two results side by side.
 template <typename TO, int THREADS, int VPT, int MAXP, bool PAIR>
 __global__ void __launch_bounds__(THREADS)
-stream_norm_vec_kernel(float *__restrict__ resid, const float *__restrict__ delta, int n_parts, size_t part_stride,
+stream_norm_vec_kernel(float *resid, const float *delta, int n_parts, size_t part_stride,
                        const float *__restrict__ col_bias, ResultNorms rn, const float *__restrict__ weight, float eps,
-                       TO *__restrict__ out, const int *__restrict__ rows, float *__restrict__ resid_out, int hidden) {
+                       TO *__restrict__ out, const int *rows, float *__restrict__ resid_out, int hidden) {
   __shared__ float scratch[2 * (THREADS / 32 + 1)];
   grid_dependents_launch();
   const int n4 = hidden / 4, i = blockIdx.x;
@@ -725,8 +730,8 @@ LLM_EXPORT int llm_stream_norm(float *resid, const float *delta, int n_parts, lo
 // z 32-bit (the sum of z_parts partial products), table [vocab, table_width] and out in the engine's type.
 template <typename T>
 __global__ void __launch_bounds__(256)
-token_gate_kernel(const float *__restrict__ z, long long ldz, int z_parts, long long z_stride, const T *__restrict__ table, long long table_width, int offset, int dim,
-                  const int *__restrict__ ids, const int *__restrict__ rows, T *__restrict__ out, int ldo, size_t total) {
+token_gate_kernel(const float *z, long long ldz, int z_parts, long long z_stride, const T *__restrict__ table, long long table_width, int offset, int dim,
+                  const int *ids, const int *rows, T *__restrict__ out, int ldo, size_t total) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
@@ -774,9 +779,9 @@ LLM_EXPORT int llm_add_rmsnorm(float *resid, const void *delta, int delta_dtype,
 // the block's fixed order).
 template <typename TD, typename TO, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-add_layernorm_kernel(float *__restrict__ resid, const TD *__restrict__ delta, int n_parts, size_t part_stride,
+add_layernorm_kernel(float *resid, const TD *delta, int n_parts, size_t part_stride,
                      const float *__restrict__ weight, const float *__restrict__ bias, float eps, TO *__restrict__ out,
-                     const int *__restrict__ rows, int hidden) {
+                     const int *rows, int hidden) {
   extern __shared__ float row_buf[];   // hidden floats
   __shared__ float scratch[THREADS / 32 + 1];
   grid_dependents_launch();
@@ -811,9 +816,9 @@ add_layernorm_kernel(float *__restrict__ resid, const TD *__restrict__ delta, in
 // the general kernel's only in which thread owns which columns; a row's result does not depend on the launch.
 template <typename TD, typename TO, int THREADS, int VPT, int MAXP>
 __global__ void __launch_bounds__(THREADS)
-add_layernorm_vec_kernel(float *__restrict__ resid, const TD *__restrict__ delta, int n_parts, size_t part_stride,
+add_layernorm_vec_kernel(float *resid, const TD *delta, int n_parts, size_t part_stride,
                          const float *__restrict__ weight, const float *__restrict__ bias, float eps, TO *__restrict__ out,
-                         const int *__restrict__ rows, int hidden) {
+                         const int *rows, int hidden) {
   __shared__ float scratch[THREADS / 32 + 1];
   grid_dependents_launch();
   const int i = blockIdx.x;
@@ -955,9 +960,9 @@ LLM_EXPORT int llm_add_layernorm(float *resid, const void *delta, int delta_dtyp
 // own channels only.
 template <typename TD, typename TO, int THREADS, int VPT, int MAXP>
 __global__ void __launch_bounds__(THREADS)
-add_layernorm_conv_kernel(float *__restrict__ resid, const TD *__restrict__ delta, int n_parts, size_t part_stride,
+add_layernorm_conv_kernel(float *resid, const TD *delta, int n_parts, size_t part_stride,
                           const float *__restrict__ weight, const float *__restrict__ bias, float eps, TO *__restrict__ out,
-                          int hidden, const float *__restrict__ conv_w, TO *__restrict__ state, const int *__restrict__ seq_slot,
+                          int hidden, const float *__restrict__ conv_w, TO *state, const int *seq_slot,
                           int taps) {
   constexpr int MAX_KEEP = 7;            // taps - 1 of the longest convolution
   __shared__ float scratch[THREADS / 32 + 1];
@@ -1100,8 +1105,8 @@ LLM_EXPORT int llm_add_layernorm_conv(float *resid, const void *delta, int delta
 // out[i] = resid[rows[i]] + sum_p delta[p][rows[i]] (32-bit, parts in index order): the residual
 // stream of the rows that anything still reads, when the others are done with.
 template <typename TD>
-__global__ void gather_rows_add_kernel(const float *__restrict__ resid, const TD *__restrict__ delta, int n_parts,
-                                       size_t part_stride, const int *__restrict__ rows, float *__restrict__ out, int hidden,
+__global__ void gather_rows_add_kernel(const float *resid, const TD *delta, int n_parts,
+                                       size_t part_stride, const int *rows, float *__restrict__ out, int hidden,
                                        const float *__restrict__ col_scale, const float *__restrict__ col_bias) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1146,7 +1151,7 @@ LLM_EXPORT int llm_gather_rows_add(const float *resid, const void *delta, int de
 // out[t, i] = silu(gu[t, i]) * gu[t, inter + i], silu(a) = a / (1 + exp(-a)).  TI is the
 // type of the stacked gate|up product (32-bit when the product gives that), T of out.
 template <typename TI, typename T>
-__global__ void swiglu_kernel(const TI *__restrict__ gu, T *__restrict__ out, int inter, size_t total) {
+__global__ void swiglu_kernel(const TI *gu, T *__restrict__ out, int inter, size_t total) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -1161,7 +1166,7 @@ __global__ void swiglu_kernel(const TI *__restrict__ gu, T *__restrict__ out, in
 
 // Four values per thread (widths that are a multiple of 4, 16-byte aligned rows).
 template <typename TI, typename T>
-__global__ void swiglu_vec_kernel(const TI *__restrict__ gu, T *__restrict__ out, int inter4, size_t total4) {
+__global__ void swiglu_vec_kernel(const TI *gu, T *__restrict__ out, int inter4, size_t total4) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total4;
@@ -1214,7 +1219,7 @@ __device__ __forceinline__ float clamped_glu_one(float g, float u, float limit, 
 }
 
 template <typename TI, typename T>
-__global__ void clamped_glu_kernel(const TI *__restrict__ gu, long long ld, const float *__restrict__ bias, T *__restrict__ out,
+__global__ void clamped_glu_kernel(const TI *gu, long long ld, const float *__restrict__ bias, T *__restrict__ out,
                                    int inter, size_t total, float limit, float slope, float up_shift) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1229,7 +1234,7 @@ __global__ void clamped_glu_kernel(const TI *__restrict__ gu, long long ld, cons
 
 // Four values per thread (widths that are a multiple of 4, 16-byte aligned rows).
 template <typename TI, typename T>
-__global__ void clamped_glu_vec_kernel(const TI *__restrict__ gu, long long ld, const float *__restrict__ bias, T *__restrict__ out,
+__global__ void clamped_glu_vec_kernel(const TI *gu, long long ld, const float *__restrict__ bias, T *__restrict__ out,
                                        int inter4, size_t total4, float limit, float slope, float up_shift) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1277,7 +1282,7 @@ LLM_EXPORT int llm_clamped_glu(int in_dtype, int dtype, const void *gu, long lon
 
 // ---------------------------------------------------------------- scaling of rows and logits
 // x *= scale over n values: the token rows of an architecture that scales its embedding.
-__global__ void scale_rows_kernel(float *__restrict__ x, long long n, float scale) {
+__global__ void scale_rows_kernel(float *x, long long n, float scale) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -1295,7 +1300,7 @@ LLM_EXPORT int llm_scale_rows(float *x, long long n, float scale, cudaStream_t s
 }
 
 // logit = logit * scale, then, with a positive cap, cap * tanh(logit / cap), in 32-bit.
-__global__ void logit_transform_kernel(float *__restrict__ x, long long n, float scale, float cap) {
+__global__ void logit_transform_kernel(float *x, long long n, float scale, float cap) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -1359,8 +1364,8 @@ LLM_EXPORT int llm_random_fill(void *out, int dtype, long long n, unsigned long 
 // the type of out: the input of a projection that mixes the residual stream with a second tensor
 // of the same shape (the token rows, for a model that feeds them to every pass of a loop).
 template <typename TO>
-__global__ void concat_stream_kernel(const float *__restrict__ resid, const float *__restrict__ delta, int n_parts,
-                                     size_t part_stride, const float *__restrict__ other, TO *__restrict__ out,
+__global__ void concat_stream_kernel(const float *resid, const float *delta, int n_parts,
+                                     size_t part_stride, const float *other, TO *__restrict__ out,
                                      int hidden, size_t total) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1398,7 +1403,7 @@ LLM_EXPORT int llm_concat_stream(const float *resid, const float *delta, int n_p
 // x[t, h * dv + c] *= sigmoid(gate[t * gate_stride + h]): the output gate of an attention whose
 // kernel does not apply it itself.  The gate is 32-bit (a column block of the stacked product).
 template <typename T>
-__global__ void head_gate_kernel(T *__restrict__ x, long long ld, const float *__restrict__ gate, long long gate_stride,
+__global__ void head_gate_kernel(T *x, long long ld, const float *gate, long long gate_stride,
                                  int n_heads, int dv, size_t total) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1414,7 +1419,7 @@ __global__ void head_gate_kernel(T *__restrict__ x, long long ld, const float *_
 
 // Four channels to a thread (head widths that are a multiple of 4, 8-byte aligned rows).
 template <typename T>
-__global__ void head_gate_vec_kernel(T *__restrict__ x, long long ld, const float *__restrict__ gate, long long gate_stride,
+__global__ void head_gate_vec_kernel(T *x, long long ld, const float *gate, long long gate_stride,
                                      int n_heads, int dv4, size_t total4) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1431,7 +1436,7 @@ __global__ void head_gate_vec_kernel(T *__restrict__ x, long long ld, const floa
 
 // A gate per channel: x[t, c] *= sigmoid(gate[t * gate_stride + c]), four channels to a thread.
 template <typename T>
-__global__ void channel_gate_vec_kernel(T *__restrict__ x, long long ld, const float *__restrict__ gate, long long gate_stride,
+__global__ void channel_gate_vec_kernel(T *x, long long ld, const float *gate, long long gate_stride,
                                         int width4, size_t total4) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -1507,11 +1512,11 @@ LLM_EXPORT int llm_head_gate(void *x, int dtype, long long ld, const float *gate
 constexpr int HYPER_MAX_STREAMS = 16;
 template <typename TO, int THREADS, int VEC, int MAXS>       // MAXS >= S: how many copies the unrolled loops provide for
 __global__ void __launch_bounds__(THREADS)
-hyper_mix_norm_kernel(const float *__restrict__ x_in, long long in_stride, float *__restrict__ x_out, long long out_stride, int S,
-                      const float *__restrict__ delta, int n_parts, size_t part_stride, const float *__restrict__ col_scale,
+hyper_mix_norm_kernel(const float *x_in, long long in_stride, float *x_out, long long out_stride, int S,
+                      const float *delta, int n_parts, size_t part_stride, const float *__restrict__ col_scale,
                       const float *__restrict__ col_bias, const float *__restrict__ mix, const float *__restrict__ outw,
                       const float *__restrict__ inw, const float *__restrict__ norm_w, float eps, TO *__restrict__ out,
-                      const int *__restrict__ rows, int hidden) {
+                      const int *rows, int hidden) {
   extern __shared__ float row_buf[];   // hidden floats
   __shared__ float scratch[THREADS / 32 + 1];
   __shared__ float s_mix[MAXS * MAXS], s_out[MAXS], s_in[MAXS];
@@ -1670,9 +1675,9 @@ LLM_EXPORT int llm_add_scalar(float *x, long long n, float value, cudaStream_t s
 // resid[r, c] = resid[r, c] + (sum of delta's parts + col_bias) * col_scale + other[r, c] + vec[c]; delta, other and vec may be
 // null.  32-bit, parts in order.  A CTA a row.
 __global__ void __launch_bounds__(256)
-stream_add_kernel(float *__restrict__ resid, const float *__restrict__ delta, int n_parts, long long part_stride,
-                  const float *__restrict__ col_scale, const float *__restrict__ col_bias, const float *__restrict__ other,
-                  const float *__restrict__ vec, int hidden) {
+stream_add_kernel(float *resid, const float *delta, int n_parts, long long part_stride,
+                  const float *__restrict__ col_scale, const float *__restrict__ col_bias, const float *other,
+                  const float *vec, int hidden) {
   grid_dependents_launch();
   grid_dependency_wait();
   const size_t row = (size_t)blockIdx.x * hidden;

@@ -52,7 +52,7 @@ struct FewShape {
 };
 template <int MT>
 __global__ void __launch_bounds__(128)
-gemm_few_kernel(const float *__restrict__ A, long long lda, const float *__restrict__ W, long long ldw,
+gemm_few_kernel(const float *A, long long lda, const float *__restrict__ W, long long ldw,
                 const float *__restrict__ bias, float *__restrict__ C, long long ldc, int M, int N, int K) {
   using S = FewShape<MT>;
   constexpr int PITCH = S::PITCH, STAGES = S::STAGES;
@@ -154,7 +154,7 @@ struct TileShape {
   static constexpr size_t SMEM = RING > SUMS ? RING : SUMS;
 };
 __global__ void __launch_bounds__(256, 1)
-gemm_tile_kernel(const float *__restrict__ A, long long lda, const float *__restrict__ W, long long ldw,
+gemm_tile_kernel(const float *A, long long lda, const float *__restrict__ W, long long ldw,
                  const float *__restrict__ bias, float *__restrict__ C, long long ldc, int M, int N, int K) {
   using S = TileShape;
   constexpr int RM = S::RM, PITCH = S::PITCH, KS = S::KS, STAGES = S::STAGES, LM = RM / 4;

@@ -43,7 +43,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1
 // rows, then up rows); row r pairs with row inter + r and out is [M, inter].
 template <int NT, int MT, int UNROLL, bool SWIGLU, typename TO>
 __global__ void __launch_bounds__(GEMV_WARPS * 32)
-gemv_kernel(const __nv_bfloat16 *__restrict__ x, long long ldx, const __nv_bfloat16 *__restrict__ W,
+gemv_kernel(const __nv_bfloat16 *x, long long ldx, const __nv_bfloat16 *__restrict__ W,
             TO *__restrict__ out, long long ldo, int M, int N, int K, int k_split, int kb_per_part,
             long long part_stride) {
   constexpr int SETS = SWIGLU ? 2 : 1;
@@ -120,7 +120,7 @@ gemv_kernel(const __nv_bfloat16 *__restrict__ x, long long ldx, const __nv_bfloa
       const bool kok = k < K;
 #pragma unroll
       for (int n = 0; n < NT; ++n)
-        b[u][n] = (kok && xok[n]) ? __ldg(reinterpret_cast<const uint4 *>(xrow[n] + k)) : make_uint4(0, 0, 0, 0);
+        b[u][n] = (kok && xok[n]) ? *reinterpret_cast<const uint4 *>(xrow[n] + k) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u)

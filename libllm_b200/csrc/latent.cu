@@ -37,10 +37,10 @@ __device__ __forceinline__ void rotate_pair(const float *x, const float *cs, int
 // engine's type; cache row of the token = [rms(first kv_rank) * kv_weight | rotated last rot_dim].
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-latent_place_kernel(const float *__restrict__ proj, long long ld, int off_q, int q_rank, const float *__restrict__ q_weight,
+latent_place_kernel(const float *proj, long long ld, int off_q, int q_rank, const float *__restrict__ q_weight,
                     T *__restrict__ cq_out, long long ldq, int off_kv, int kv_rank, int rot, const float *__restrict__ kv_weight,
-                    float eps, const float *__restrict__ table, int table_rows, int interleaved, const int *__restrict__ tok_seq,
-                    const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride, T *__restrict__ cache,
+                    float eps, const float *__restrict__ table, int table_rows, int interleaved, const int *tok_seq,
+                    const int *tok_pos, const int *page_table, int pt_stride, T *__restrict__ cache,
                     int page_size) {
   __shared__ float scratch[THREADS / 32 + 1];
   grid_dependents_launch();
@@ -106,9 +106,9 @@ LLM_EXPORT int llm_latent_place(int dtype, const float *proj, long long ld, int 
 constexpr int LAT_TT = 16;
 template <typename T, int THREADS, int TT, int V>
 __global__ void __launch_bounds__(THREADS)
-latent_absorb_kernel(const float *__restrict__ q, long long ldq, const T *__restrict__ w_uk, T *__restrict__ out, long long ldo,
+latent_absorb_kernel(const float *q, long long ldq, const T *__restrict__ w_uk, T *__restrict__ out, long long ldo,
                      int n_tokens, int d, int rot, int kv_rank, const float *__restrict__ table, int table_rows, int interleaved,
-                     const int *__restrict__ tok_pos) {
+                     const int *tok_pos) {
   extern __shared__ float qs[];                        // [TT][d]
   struct alignas(sizeof(T) * V) Piece { T v[V]; };
   constexpr int ROWS = sizeof(T) == 2 ? 64 : 32;       // rows of w_uk held at once
@@ -218,8 +218,8 @@ LLM_EXPORT int llm_latent_absorb(int dtype, const float *q, long long ldq, const
 constexpr int LAT_ET = 8;
 template <typename T, int THREADS, int ET>
 __global__ void __launch_bounds__(THREADS)
-latent_expand_kernel(const T *__restrict__ x, long long ldx, const T *__restrict__ w_uv, T *__restrict__ out, long long ldo, int n_tokens,
-                     int kv_rank, int dv, const float *__restrict__ gate, long long gate_stride) {
+latent_expand_kernel(const T *x, long long ldx, const T *__restrict__ w_uv, T *__restrict__ out, long long ldo, int n_tokens,
+                     int kv_rank, int dv, const float *gate, long long gate_stride) {
   extern __shared__ float xs[];                        // [ET][kv_rank]
   constexpr int HELD = 16;
   grid_dependents_launch();

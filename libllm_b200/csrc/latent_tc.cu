@@ -31,8 +31,8 @@ constexpr int LT_BN = 64;                // keys per tile
 // ---------------------------------------------------------------- the step's rows, out of the cache
 // c_out [T, kv_rank] and kr_out [T, rot] = the cached rows of the step's tokens (whoever appended them).
 __global__ void __launch_bounds__(128)
-latent_rows_kernel(const __nv_bfloat16 *__restrict__ cache, int page_size, int row, int kv_rank, const int *__restrict__ tok_seq,
-                   const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride,
+latent_rows_kernel(const __nv_bfloat16 *cache, int page_size, int row, int kv_rank, const int *tok_seq,
+                   const int *tok_pos, const int *page_table, int pt_stride,
                    __nv_bfloat16 *__restrict__ c_out, __nv_bfloat16 *__restrict__ kr_out) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -60,8 +60,8 @@ LLM_EXPORT int llm_latent_rows(const void *cache, int page_size, int row, int kv
 // position.  Table row = [cosines (rot/2) | sines (rot/2)]; pair i is channels (2i, 2i+1) when interleaved, else
 // (i, i + rot/2).
 __global__ void __launch_bounds__(256)
-latent_rotate_q_kernel(const float *__restrict__ q, long long ldq, __nv_bfloat16 *__restrict__ out, long long ldo, int n_heads, int d,
-                       int rot, const float *__restrict__ table, int table_rows, int interleaved, const int *__restrict__ tok_pos) {
+latent_rotate_q_kernel(const float *q, long long ldq, __nv_bfloat16 *__restrict__ out, long long ldo, int n_heads, int d,
+                       int rot, const float *__restrict__ table, int table_rows, int interleaved, const int *tok_pos) {
   grid_dependents_launch();
   grid_dependency_wait();
   const int t = blockIdx.x, dk = d + rot, half = rot / 2;
@@ -107,10 +107,10 @@ constexpr int LP_BM = 16 * LP_WARPS;
 
 template <int DVP>
 __global__ void __launch_bounds__(LP_WARPS * 32)
-latent_prefill_kernel(const __nv_bfloat16 *__restrict__ q, long long ldq, const __nv_bfloat16 *__restrict__ kv, long long ldkv,
-                      const __nv_bfloat16 *__restrict__ kr, __nv_bfloat16 *__restrict__ out, long long ldo,
-                      const int *__restrict__ seq_start, int n_heads, int d, int rot, int dv, float scale_log2, int window,
-                      const float *__restrict__ null_scores, const float *__restrict__ gate, long long gate_stride) {
+latent_prefill_kernel(const __nv_bfloat16 *q, long long ldq, const __nv_bfloat16 *kv, long long ldkv,
+                      const __nv_bfloat16 *kr, __nv_bfloat16 *__restrict__ out, long long ldo,
+                      const int *seq_start, int n_heads, int d, int rot, int dv, float scale_log2, int window,
+                      const float *__restrict__ null_scores, const float *gate, long long gate_stride) {
   constexpr int LDV = DVP + 8;
   constexpr int VCH = DVP / 8;
   constexpr int NT = LT_BN / 8;
@@ -369,8 +369,8 @@ static __host__ __device__ inline int latent_rowp(int row) { return (row + 15) /
 
 template <int MAXR>                      // kv_rank <= MAXR; a warp owns MAXR / 4 value channels
 __global__ void __launch_bounds__(LD_WARPS * 32)
-latent_decode_kernel(const __nv_bfloat16 *__restrict__ qa, long long ldq, const __nv_bfloat16 *__restrict__ cache, int page_size,
-                     const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride,
+latent_decode_kernel(const __nv_bfloat16 *qa, long long ldq, const __nv_bfloat16 *cache, int page_size,
+                     const int *tok_seq, const int *tok_pos, const int *page_table, int pt_stride,
                      int n_heads, int row, int kv_rank, int n_splits, float scale_log2, __nv_bfloat16 *__restrict__ out, long long ldo,
                      float *__restrict__ ws_o, float *__restrict__ ws_ml, int window, const float *__restrict__ null_scores) {
   constexpr int SL = MAXR / 4;           // value channels of a warp
@@ -591,7 +591,7 @@ latent_decode_kernel(const __nv_bfloat16 *__restrict__ qa, long long ldq, const 
 // weights go through shared memory once, so that the loads of the partial sums are independent of one another.
 constexpr int LJ_MAX = 64;               // runs at most
 __global__ void __launch_bounds__(128)
-latent_join_kernel(const float *__restrict__ ws_o, const float *__restrict__ ws_ml, int n_splits, int kv_rank,
+latent_join_kernel(const float *ws_o, const float *ws_ml, int n_splits, int kv_rank,
                    __nv_bfloat16 *__restrict__ out, long long ldo, int n_heads, const float *__restrict__ null_scores) {
   __shared__ float w[LJ_MAX];
   __shared__ float inv_s;

@@ -49,8 +49,8 @@ __device__ __forceinline__ float gated_unit(float g, float u, int act, const Glu
 
 // ---------------------------------------------------------------- choice of experts
 // One warp per token.  score_kind 0: sigmoid, 1: softmax over all experts.
-__global__ void moe_route_kernel(const float *__restrict__ logits, long long ld, int n_tokens, int n_experts, int top,
-                                 int score_kind, int renormalize, int *__restrict__ chosen, float *__restrict__ weight) {
+__global__ void moe_route_kernel(const float *logits, long long ld, int n_tokens, int n_experts, int top,
+                                 int score_kind, int renormalize, int *chosen, float *weight) {
   grid_dependents_launch();
   grid_dependency_wait();
   const int lane = threadIdx.x & 31;
@@ -128,8 +128,8 @@ struct RouteRule {
   float norm_eps, route_scale;
 };
 // one token by one warp; c [n_experts] and gs [n_groups] in shared memory are the warp's own
-__device__ __forceinline__ void route_token(const float *__restrict__ z, const RouteRule &R, float *c, float *gs, int lane, int *__restrict__ chosen,
-                                            float *__restrict__ weight) {
+__device__ __forceinline__ void route_token(const float *z, const RouteRule &R, float *c, float *gs, int lane, int *chosen,
+                                            float *weight) {
   const int n_experts = R.n_experts, top = R.top;
   float zmax = -INFINITY, denom = 1.f;
   if (R.score_kind == 1) {
@@ -232,8 +232,8 @@ __device__ __forceinline__ void route_token(const float *__restrict__ z, const R
   }
 }
 
-__global__ void moe_route_grouped_kernel(const float *__restrict__ logits, long long ld, int n_tokens, RouteRule R, int *__restrict__ chosen,
-                                         float *__restrict__ weight) {
+__global__ void moe_route_grouped_kernel(const float *logits, long long ld, int n_tokens, RouteRule R, int *chosen,
+                                         float *weight) {
   extern __shared__ float route_sh[];            // per warp: c [E], group scores [n_groups]
   grid_dependents_launch();
   grid_dependency_wait();
@@ -266,8 +266,8 @@ LLM_EXPORT int llm_moe_route_grouped(const float *logits, long long ld, int n_to
 
 // out[p, t, :] = x[p, t, :] * sigmoid(gate[t * gate_stride]) for every part p (32-bit rows; parts x_stride and out_stride
 // floats apart): a feed-forward's result, whole or in partial products, weighed by one number per token.
-__global__ void row_gate_kernel(const float *__restrict__ x, long long x_stride, float *__restrict__ out, long long out_stride,
-                                const float *__restrict__ gate, long long gate_stride, int cols, long long total) {
+__global__ void row_gate_kernel(const float *x, long long x_stride, float *__restrict__ out, long long out_stride,
+                                const float *gate, long long gate_stride, int cols, long long total) {
   grid_dependents_launch();
   grid_dependency_wait();
   const float *xp = x + (size_t)blockIdx.y * x_stride;
@@ -297,8 +297,8 @@ LLM_EXPORT int llm_row_gate(const float *x, long long x_stride, float *out, long
 // in; no result depends on it.  Rows of identity experts (chosen >= n_experts) get no place.
 // By all threads of a block; counts and cursor [E] in shared memory.
 template <bool STABLE = false>
-__device__ __forceinline__ void sort_rows(const int *chosen, int n_rows, int n_experts, int tile_rows, int *__restrict__ offsets,
-                                          int *__restrict__ perm, int *__restrict__ tiles, int *counts, int *cursor) {
+__device__ __forceinline__ void sort_rows(const int *chosen, int n_rows, int n_experts, int tile_rows, int *offsets,
+                                          int *perm, int *tiles, int *counts, int *cursor) {
   for (int e = threadIdx.x; e < n_experts; e += blockDim.x) counts[e] = 0;
   __syncthreads();
   for (int r = threadIdx.x; r < n_rows; r += blockDim.x)
@@ -349,8 +349,8 @@ __device__ __forceinline__ void sort_rows(const int *chosen, int n_rows, int n_e
 }
 
 __global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int *__restrict__ chosen, int n_rows, int n_experts, int tile_rows, int *__restrict__ offsets,
-                int *__restrict__ perm, int *__restrict__ tiles) {
+moe_sort_kernel(const int *chosen, int n_rows, int n_experts, int tile_rows, int *offsets,
+                int *perm, int *tiles) {
   extern __shared__ int sh[];                  // counts [E], cursor [E]
   grid_dependents_launch();
   grid_dependency_wait();
@@ -370,7 +370,7 @@ LLM_EXPORT int llm_moe_tile_rows() { return 64; }
 
 // ---------------------------------------------------------------- both products, a CTA per row
 template <typename T>
-__device__ __forceinline__ float dot_cols(const T *__restrict__ w, const float *__restrict__ x, int n, int lane) {
+__device__ __forceinline__ float dot_cols(const T *__restrict__ w, const float *x, int n, int lane) {
   float acc = 0.f;
   for (int c = lane; c < n; c += 32) acc = fmaf(to_float(w[c]), x[c], acc);
   return warp_sum(acc);
@@ -380,8 +380,8 @@ __device__ __forceinline__ float dot_cols(const T *__restrict__ w, const float *
 // weight_on 0: input, 1: output.
 template <typename T>
 __global__ void __launch_bounds__(256)
-moe_rows_kernel(const T *__restrict__ x, long long ldx, const T *__restrict__ up, const T *__restrict__ down,
-                const int *__restrict__ chosen, const float *__restrict__ weight, int n_tokens, int top, int width, int ff,
+moe_rows_kernel(const T *x, long long ldx, const T *__restrict__ up, const T *__restrict__ down,
+                const int *chosen, const float *weight, int n_tokens, int top, int width, int ff,
                 int act, int weight_on, int gated, int n_experts, GluShape glu, float *__restrict__ out) {
   extern __shared__ float shf[];               // x row [width], hidden [ff]
   float *xs = shf, *hs = shf + width;
@@ -448,13 +448,13 @@ LLM_EXPORT int llm_moe_rows(int dtype, const void *x, long long ldx, const void 
 // ---------------------------------------------------------------- identity experts alone
 // out[choice, token] = weight * x[token] for every row whose choice is no expert (tokens' rows in eights where they allow it).
 template <typename T>
-__device__ __forceinline__ void identity_row(const T *__restrict__ x, float w, float *__restrict__ o, int c0, int width) {
+__device__ __forceinline__ void identity_row(const T *x, float w, float *__restrict__ o, int c0, int width) {
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     if (c0 + i < width) o[c0 + i] = w * to_float(x[c0 + i]);
 }
-__global__ void moe_identity_kernel(const __nv_bfloat16 *__restrict__ x, long long ldx, const int *__restrict__ chosen,
-                                    const float *__restrict__ weight, int n_tokens, int n_experts, int top, int width,
+__global__ void moe_identity_kernel(const __nv_bfloat16 *x, long long ldx, const int *chosen,
+                                    const float *weight, int n_tokens, int n_experts, int top, int width,
                                     float *__restrict__ out) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -481,9 +481,9 @@ constexpr int GLD = GK + GPAD;                 // 40 values = 80 bytes a row: ld
 // second == 0: A = x, arow = perm[place] / top; C -> mid[place, n] = bfloat16(act and weight applied).
 // second == 1: A = mid, arow = place;           C -> out[perm % top][perm / top][n], 32-bit.
 __global__ void __launch_bounds__(256)
-moe_grouped_kernel(const __nv_bfloat16 *__restrict__ A, long long lda, const __nv_bfloat16 *__restrict__ W, int N, int K,
-                   const int *__restrict__ offsets, const int *__restrict__ perm, const int *__restrict__ tiles,
-                   const float *__restrict__ weight, int n_tokens, int top, int act, int weight_on, int second, int gated, GluShape glu,
+moe_grouped_kernel(const __nv_bfloat16 *A, long long lda, const __nv_bfloat16 *__restrict__ W, int N, int K,
+                   const int *offsets, const int *perm, const int *tiles,
+                   const float *weight, int n_tokens, int top, int act, int weight_on, int second, int gated, GluShape glu,
                    __nv_bfloat16 *__restrict__ mid, float *__restrict__ out) {
   __shared__ __align__(16) __nv_bfloat16 As[GSTAGES][GM][GLD];
   __shared__ __align__(16) __nv_bfloat16 Bs[GSTAGES][GN][GLD];
@@ -625,7 +625,7 @@ LLM_EXPORT int llm_moe_grouped_supports(int width, int ff) { return width % 8 ==
 
 // ---------------------------------------------------------------- an activation over rows
 template <typename TI, typename T>
-__global__ void activation_kernel(const TI *__restrict__ in, T *__restrict__ out, size_t n, int act) {
+__global__ void activation_kernel(const TI *in, T *__restrict__ out, size_t n, int act) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -634,7 +634,7 @@ __global__ void activation_kernel(const TI *__restrict__ in, T *__restrict__ out
 
 // Four values to a thread (counts that are multiples of 4, 16-byte aligned).
 template <typename TI, typename T>
-__global__ void activation_vec_kernel(const TI *__restrict__ in, T *__restrict__ out, size_t n4, int act) {
+__global__ void activation_vec_kernel(const TI *in, T *__restrict__ out, size_t n4, int act) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
@@ -680,9 +680,9 @@ LLM_EXPORT int llm_activation(int in_dtype, int dtype, const void *in, void *out
 // xs[place] = x[perm[place] / top], 16 bytes to a thread: the operand of the tensor-memory form of the first
 // product (csrc/moe_tc.cu), whose loads want the rows of a tile one behind the other.  With `chosen` (some rows are identity
 // experts') only the first offsets[n_experts] places hold rows, and the identity experts' results go to `out` on the way.
-__global__ void moe_gather_kernel(const uint4 *__restrict__ x, long long ldx16, const int *__restrict__ perm, int top,
-                                  int width16, size_t total, uint4 *__restrict__ xs, const int *__restrict__ chosen,
-                                  const int *__restrict__ offsets, const float *__restrict__ weight, int n_experts, int n_tokens,
+__global__ void moe_gather_kernel(const uint4 *x, long long ldx16, const int *perm, int top,
+                                  int width16, size_t total, uint4 *__restrict__ xs, const int *chosen,
+                                  const int *offsets, const float *weight, int n_experts, int n_tokens,
                                   float *__restrict__ out) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -721,8 +721,8 @@ LLM_EXPORT int llm_moe_gather_identity(const void *x, long long ldx, const int *
 // are added here.
 constexpr int MOE_PLAN_ROWS = 64, MOE_PLAN_WARPS = 32;
 __global__ void __launch_bounds__(MOE_PLAN_WARPS * 32)
-moe_plan_kernel(const float *__restrict__ logits, long long ld, int z_parts, long long z_stride, int n_tokens, RouteRule R, int n_experts, int tile_rows,
-                const uint4 *__restrict__ x, long long ldx16, int width16, int *chosen, float *weight, int *offsets, int *perm, int *tiles,
+moe_plan_kernel(const float *logits, long long ld, int z_parts, long long z_stride, int n_tokens, RouteRule R, int n_experts, int tile_rows,
+                const uint4 *x, long long ldx16, int width16, int *chosen, float *weight, int *offsets, int *perm, int *tiles,
                 uint4 *__restrict__ xs, float *__restrict__ out) {
   extern __shared__ float plan_sh[];             // per warp: z and c [choices], group scores; then counts [E], cursor [E], correction
   __shared__ int chosen_s[MOE_PLAN_ROWS], perm_s[MOE_PLAN_ROWS];

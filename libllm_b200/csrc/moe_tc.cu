@@ -58,8 +58,8 @@ struct MtShape {
 template <int TN, int ACT, bool GATED>
 __global__ void __launch_bounds__(MT_THREADS, 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, int N, int K,
-              const int *__restrict__ offsets, const int *__restrict__ perm, const int *__restrict__ tiles,
-              const float *__restrict__ weight, int n_tokens, int top, int weight_on, GluShape glu,
+              const int *offsets, const int *perm, const int *tiles,
+              const float *weight, int n_tokens, int top, int weight_on, GluShape glu,
               __nv_bfloat16 *__restrict__ mid, float *__restrict__ out, int *status) {
   using S = MtShape<TN>;
   constexpr int STAGES = S::STAGES;

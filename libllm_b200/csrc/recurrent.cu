@@ -81,9 +81,9 @@ __device__ __forceinline__ void conv_store(T *p, const ConvVec<T, V> &r) {
 constexpr int CONV_AHEAD = 4;
 template <typename T, int V, int N>
 __global__ void __launch_bounds__(CONV_THREADS)
-causal_conv_kernel(const T *__restrict__ h, long long ldh, T *__restrict__ out, long long ldo, const float *__restrict__ weight,
-                   T *__restrict__ state, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
-                   const int *__restrict__ seq_start, const int *__restrict__ seq_past, const int *__restrict__ seq_slot,
+causal_conv_kernel(const T *h, long long ldh, T *__restrict__ out, long long ldo, const float *__restrict__ weight,
+                   T *state, const int *tok_seq, const int *tok_pos,
+                   const int *seq_start, const int *seq_past, const int *seq_slot,
                    int n_tokens, int width, int taps, int n_chunks, int chunk_rows, int mode) {
   using Vec = ConvVec<T, V>;
   grid_dependents_launch();
@@ -216,7 +216,7 @@ constexpr int DP_TOKENS = 32;                        // tokens of a CTA
 // token and three to eight with four (168 -> 104 us for 2,841 tokens of 32 heads of 64, rank 64).  One where a decay input is too wide for four.
 template <int DP_TT>
 __global__ void __launch_bounds__(DP_WARPS * 32)
-delta_prepare_kernel(const float *__restrict__ proj, long long ld, int off_k, int off_a, int off_x1, int rank,
+delta_prepare_kernel(const float *proj, long long ld, int off_k, int off_a, int off_x1, int rank,
                      const float *__restrict__ w2, const float *__restrict__ w0, const float *__restrict__ a_bias,
                      float decay_scale, float key_eps, int n_tokens, int n_heads, int d, int w2_shared,
                      float *__restrict__ prep) {
@@ -367,9 +367,9 @@ __device__ __forceinline__ float delta_token(float (&S)[ROWS], const float *vecs
 
 template <int DMAX, int LANES, bool VEC>
 __global__ void __launch_bounds__(DR_THREADS + 32)
-delta_rule_kernel(const float *__restrict__ proj, long long ld, int off_r, int off_k, int off_v,
-                  const float *__restrict__ prep, float *__restrict__ state, float *__restrict__ out, long long ldo,
-                  const int *__restrict__ seq_start, const int *__restrict__ seq_slot, int n_heads, int d, int dv) {
+delta_rule_kernel(const float *proj, long long ld, int off_r, int off_k, int off_v,
+                  const float *prep, float *state, float *__restrict__ out, long long ldo,
+                  const int *seq_start, const int *seq_slot, int n_heads, int d, int dv) {
   constexpr int ROWS = DMAX / LANES;                 // rows of a column held by one thread
   constexpr int COLS = DR_THREADS / LANES;           // columns of a CTA
   constexpr int PAD = ROWS + 4;                      // a lane's share of a vector, padded: the lanes' loads fall on different banks
@@ -541,10 +541,10 @@ LLM_EXPORT int llm_delta_scan(const float *proj, long long ld, int off_r, int of
 // arithmetic, with all of the head's columns in this CTA), the norm over the head, its weight and the gate.
 template <int DMAX, int LANES, typename TO>
 __global__ void __launch_bounds__(DMAX *LANES)
-delta_step_kernel(const float *__restrict__ proj, long long ld, int off_r, int off_k, int off_v, int off_g, int off_a, int off_x1,
+delta_step_kernel(const float *proj, long long ld, int off_r, int off_k, int off_v, int off_g, int off_a, int off_x1,
                   int rank, const float *__restrict__ w2, const float *__restrict__ w0, const float *__restrict__ a_bias,
-                  float decay_scale, float key_eps, const float *__restrict__ norm_w, float eps, float *__restrict__ state,
-                  TO *__restrict__ out, long long ldo, const int *__restrict__ seq_slot, int n_heads, int d, int w2_shared) {
+                  float decay_scale, float key_eps, const float *__restrict__ norm_w, float eps, float *state,
+                  TO *__restrict__ out, long long ldo, const int *seq_slot, int n_heads, int d, int w2_shared) {
   constexpr int ROWS = DMAX / LANES, PAD = ROWS + 4, VLEN = LANES * PAD, THREADS = DMAX * LANES;
   __shared__ __align__(16) float vecs[5 * VLEN];
   __shared__ float vals[DMAX], outs[DMAX], red[2];
@@ -655,7 +655,7 @@ LLM_EXPORT int llm_delta_step(const float *proj, long long ld, int off_r, int of
 // One warp per (token, head).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128)
-head_norm_gate_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ weight, const float *__restrict__ gate,
+head_norm_gate_kernel(const float *x, long long ldx, const float *__restrict__ weight, const float *gate,
                       long long gate_stride, float eps, int n_tokens, int n_heads, int dv, T *__restrict__ out, long long ldo) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -759,7 +759,7 @@ constexpr int CD_TT = 4;
 __device__ __forceinline__ float softplus32(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 __global__ void __launch_bounds__(CD_THREADS)
-channel_delta_prepare_kernel(float *__restrict__ cv, long long ldc, const float *__restrict__ proj, long long ld, int off_b, int off_a1,
+channel_delta_prepare_kernel(float *cv, long long ldc, const float *proj, long long ld, int off_b, int off_a1,
                              int rank_a, int off_g1, int rank_g, const float *__restrict__ a2, const float *__restrict__ dt_bias,
                              const float *__restrict__ a_log, const float *__restrict__ g2, float key_eps, float *__restrict__ prep,
                              float *__restrict__ gate, int n_tokens, int n_heads, int n_kv, int d, int dv) {

@@ -20,11 +20,11 @@ LLM_DEFINE_LAST_ERROR(llm_rope_last_error)
 // give that, so that q and k are rounded once, after the rotation); T: type of the
 // rotated queries and of the cache.
 template <typename TI, typename T>
-__global__ void rope_cache_write_kernel(const TI *__restrict__ qkv, long long row_stride,
+__global__ void rope_cache_write_kernel(const TI *qkv, long long row_stride,
                                         T *__restrict__ q_out, long long q_stride, int n_heads,
                                         int n_kv, int d, const float *__restrict__ table,
-                                        int table_rows, int rot_dim, const int *__restrict__ tok_seq,
-                                        const int *__restrict__ tok_pos, const int *__restrict__ page_table,
+                                        int table_rows, int rot_dim, const int *tok_seq,
+                                        const int *tok_pos, const int *page_table,
                                         int pt_stride, T *__restrict__ kcache, T *__restrict__ vcache,
                                         int page_size) {
   grid_dependents_launch();
@@ -66,10 +66,10 @@ __global__ void rope_cache_write_kernel(const TI *__restrict__ qkv, long long ro
 // page are looked up once per token.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(256)
-rope_cache_write_vec_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict__ q_out,
+rope_cache_write_vec_kernel(const TI *qkv, long long row_stride, T *__restrict__ q_out,
                             long long q_stride, int n_heads, int n_kv, int d, const float *__restrict__ table,
-                            int table_rows, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
-                            const int *__restrict__ page_table, int pt_stride, T *__restrict__ kcache,
+                            int table_rows, const int *tok_seq, const int *tok_pos,
+                            const int *page_table, int pt_stride, T *__restrict__ kcache,
                             T *__restrict__ vcache, int page_size, int n_slots) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -165,11 +165,11 @@ LLM_EXPORT int llm_rope_cache_write(int in_dtype, int dtype, const void *qkv, lo
 // 32-bit; a sum's order is fixed by the thread count, not by the batch.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(256)
-qk_place_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict__ q_out, long long q_stride,
+qk_place_kernel(const TI *qkv, long long row_stride, T *__restrict__ q_out, long long q_stride,
                 int n_heads, int n_kv, int d, int dv, const float *__restrict__ q_norm,
                 const float *__restrict__ k_norm, float eps, const float *__restrict__ table, int table_rows,
-                int rot_dim, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
-                const int *__restrict__ page_table, int pt_stride, T *__restrict__ kcache,
+                int rot_dim, const int *tok_seq, const int *tok_pos,
+                const int *page_table, int pt_stride, T *__restrict__ kcache,
                 T *__restrict__ vcache, int page_size, int write_cache) {
   __shared__ float scratch[256 / 32 + 1];
   grid_dependents_launch();
@@ -241,11 +241,11 @@ qk_place_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict_
 // rotated width of 8) and 16-byte aligned rows: both sums of squares go through one reduction.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(256)
-qk_place_vec_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict__ q_out, long long q_stride,
+qk_place_vec_kernel(const TI *qkv, long long row_stride, T *__restrict__ q_out, long long q_stride,
                     int n_heads, int n_kv, int d, int dv, const float *__restrict__ q_norm,
                     const float *__restrict__ k_norm, float eps, const float *__restrict__ table, int table_rows,
-                    int rot_dim, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
-                    const int *__restrict__ page_table, int pt_stride, T *__restrict__ kcache,
+                    int rot_dim, const int *tok_seq, const int *tok_pos,
+                    const int *page_table, int pt_stride, T *__restrict__ kcache,
                     T *__restrict__ vcache, int page_size, int write_cache) {
   __shared__ float sq[256 / 32 + 1], sk[256 / 32 + 1];
   grid_dependents_launch();
@@ -382,9 +382,9 @@ LLM_EXPORT int llm_qk_place(int in_dtype, int dtype, const void *qkv, long long 
 // a value head at a time (sum in lane order, then the shuffle tree).
 template <typename TI, typename T, bool VEC>
 __global__ void __launch_bounds__(256)
-kv_place_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict__ q_out, long long q_stride, int n_heads,
-                int n_kv, int d, int dv, const float *__restrict__ bias, float v_eps, const int *__restrict__ tok_seq,
-                const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride, T *__restrict__ kcache,
+kv_place_kernel(const TI *qkv, long long row_stride, T *__restrict__ q_out, long long q_stride, int n_heads,
+                int n_kv, int d, int dv, const float *__restrict__ bias, float v_eps, const int *tok_seq,
+                const int *tok_pos, const int *page_table, int pt_stride, T *__restrict__ kcache,
                 T *__restrict__ vcache, int page_size, int write_cache) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -491,10 +491,10 @@ LLM_EXPORT int llm_kv_place(int in_dtype, int dtype, const void *qkv, long long 
 // copied.  One CTA a token, two neighbouring channels to a thread at a time.
 template <typename TI, typename T>
 __global__ void __launch_bounds__(256)
-rope_pairs_place_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict__ q_out, long long q_stride, int n_heads,
+rope_pairs_place_kernel(const TI *qkv, long long row_stride, T *__restrict__ q_out, long long q_stride, int n_heads,
                         int n_kv, int d, int dv, const float *__restrict__ bias, int values_from_keys,
-                        const float *__restrict__ table, int table_rows, int rot_dim, const int *__restrict__ tok_seq,
-                        const int *__restrict__ tok_pos, const int *__restrict__ page_table, int pt_stride, T *__restrict__ kcache,
+                        const float *__restrict__ table, int table_rows, int rot_dim, const int *tok_seq,
+                        const int *tok_pos, const int *page_table, int pt_stride, T *__restrict__ kcache,
                         T *__restrict__ vcache, int page_size, int write_cache) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -585,9 +585,9 @@ LLM_EXPORT int llm_rope_pairs_place(int in_dtype, int dtype, const void *qkv, lo
 // item is V consecutive pairs (or unrotated channels): V = 4 where the widths are multiples of 4 and rows lie on 16 bytes.
 template <typename TI, typename T, int LANES, int ITEMS, int V>
 __global__ void __launch_bounds__(256)
-rope_headnorm_place_kernel(const TI *__restrict__ qkv, long long row_stride, T *__restrict__ q_out, long long q_stride, int n_heads,
+rope_headnorm_place_kernel(const TI *qkv, long long row_stride, T *__restrict__ q_out, long long q_stride, int n_heads,
                            int n_kv, int d, int dv, float eps, const float *__restrict__ table, int table_rows, int rot_dim,
-                           const int *__restrict__ tok_seq, const int *__restrict__ tok_pos, const int *__restrict__ page_table,
+                           const int *tok_seq, const int *tok_pos, const int *page_table,
                            int pt_stride, T *__restrict__ kcache, T *__restrict__ vcache, int page_size, int write_cache) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -756,11 +756,11 @@ __device__ __forceinline__ void cp_store(T *p, const float (&x)[V]) {
 
 template <typename T, int V, int TAPS>
 __global__ void __launch_bounds__(CP_THREADS)
-conv_rope_place_kernel(const float *__restrict__ qkv, long long ld, const float *__restrict__ bias, const float *__restrict__ conv,
-                       int taps, float *__restrict__ state, T *__restrict__ q_out, long long q_stride, int n_heads, int n_kv, int d, int dv,
-                       const float *__restrict__ table, int table_rows, int rot_dim, const int *__restrict__ tok_seq,
-                       const int *__restrict__ tok_pos, const int *__restrict__ seq_start, const int *__restrict__ seq_past,
-                       const int *__restrict__ seq_slot, const int *__restrict__ page_table, int pt_stride, T *__restrict__ kcache,
+conv_rope_place_kernel(const float *qkv, long long ld, const float *__restrict__ bias, const float *__restrict__ conv,
+                       int taps, float *state, T *__restrict__ q_out, long long q_stride, int n_heads, int n_kv, int d, int dv,
+                       const float *__restrict__ table, int table_rows, int rot_dim, const int *tok_seq,
+                       const int *tok_pos, const int *seq_start, const int *seq_past,
+                       const int *seq_slot, const int *page_table, int pt_stride, T *__restrict__ kcache,
                        T *__restrict__ vcache, int page_size, int write_cache, int n_tokens, int n_chunks) {
   grid_dependents_launch();
   const int half = rot_dim / 2, rot_units = half / V, head_units = rot_units + (d - rot_dim) / V;

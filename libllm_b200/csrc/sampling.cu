@@ -96,7 +96,7 @@ __device__ ArgMax block_argmax(const float *row, int V, float *sv, int *si) {
   return r;
 }
 
-__global__ void __launch_bounds__(ST) argmax_kernel(const float *__restrict__ logits, long long stride,
+__global__ void __launch_bounds__(ST) argmax_kernel(const float *logits, long long stride,
                                                     int V, int *__restrict__ out) {
   __shared__ float sv[32];
   __shared__ int si[32];
@@ -204,8 +204,8 @@ __device__ int block_exclusive_scan_int(int v, int *warp_tot /*33*/, int *total)
 }
 
 __global__ void __launch_bounds__(ST)
-sample_kernel(const float *__restrict__ logits, long long stride, int V, float temperature, int top_k,
-              float top_p, const float *__restrict__ uniforms, int *__restrict__ out, int only_marked) {
+sample_kernel(const float *logits, long long stride, int V, float temperature, int top_k,
+              float top_p, const float *uniforms, int *out, int only_marked) {
   __shared__ float sv[32];
   __shared__ int si[32];
   __shared__ float fscan[33];
@@ -440,7 +440,7 @@ __device__ __forceinline__ T *in_block(T *p, unsigned rank) {
 }
 
 __global__ void __cluster_dims__(SC, 1, 1) __launch_bounds__(ST)
-argmax_cluster_kernel(const float *__restrict__ logits, long long stride, int V, int *__restrict__ out) {
+argmax_cluster_kernel(const float *logits, long long stride, int V, int *__restrict__ out) {
   __shared__ float sv[32];
   __shared__ int si[32];
   __shared__ float xmax;
@@ -467,8 +467,8 @@ argmax_cluster_kernel(const float *__restrict__ logits, long long stride, int V,
 }
 
 __global__ void __cluster_dims__(SC, 1, 1) __launch_bounds__(ST)
-sample_cluster_kernel(const float *__restrict__ logits, long long stride, int V, float temperature, int top_k,
-                      float top_p, const float *__restrict__ uniforms, int *__restrict__ out) {
+sample_cluster_kernel(const float *logits, long long stride, int V, float temperature, int top_k,
+                      float top_p, const float *uniforms, int *__restrict__ out) {
   __shared__ float sv[32];
   __shared__ int si[32];
   __shared__ float fscan[33];

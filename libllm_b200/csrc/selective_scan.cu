@@ -75,10 +75,10 @@ __device__ __forceinline__ void sc_store(T *p, const float (&x)[V]) {
 
 template <typename T, int V, int TAPS>
 __global__ void __launch_bounds__(SC_THREADS)
-short_conv_silu_kernel(const float *__restrict__ u, long long ld, const float *__restrict__ weight, const float *__restrict__ bias, int taps,
-                       float *__restrict__ state, T *__restrict__ out, long long ldo, int channels, const int *__restrict__ tok_seq,
-                       const int *__restrict__ tok_pos, const int *__restrict__ seq_start, const int *__restrict__ seq_past,
-                       const int *__restrict__ seq_slot, int n_tokens, int n_chunks) {
+short_conv_silu_kernel(const float *u, long long ld, const float *__restrict__ weight, const float *__restrict__ bias, int taps,
+                       float *state, T *__restrict__ out, long long ldo, int channels, const int *tok_seq,
+                       const int *tok_pos, const int *seq_start, const int *seq_past,
+                       const int *seq_slot, int n_tokens, int n_chunks) {
   grid_dependents_launch();
   const int c0 = (blockIdx.y * SC_THREADS + threadIdx.x) * V, keep = taps - 1;
   float w[TAPS][V], bs[V], win[TAPS][V], x[V];
@@ -225,7 +225,7 @@ __device__ __forceinline__ int first_of(int lane) {
 
 // the decays (al2) and values of a lane's states, lane + i L; states beyond N are nought and stay so
 template <int L, int NS>
-__device__ __forceinline__ void lane_states(const float *__restrict__ a_log, const float *__restrict__ st, int c, int lane, int N, bool in,
+__device__ __forceinline__ void lane_states(const float *__restrict__ a_log, const float *st, int c, int lane, int N, bool in,
                                             float (&al2)[NS], float (&S)[NS]) {
 #pragma unroll
   for (int i = 0; i < NS; ++i) {
@@ -237,11 +237,11 @@ __device__ __forceinline__ void lane_states(const float *__restrict__ a_log, con
 
 template <typename T, int L, int NS>
 __global__ void __launch_bounds__(SCAN_THREADS)
-selective_scan_kernel(const T *__restrict__ x, long long ldx, const float *__restrict__ dt_raw, long long ld_dt,
-                      const float *__restrict__ dt_bias, const float *__restrict__ bc, long long ld_bc, int off_b, int off_c,
-                      const float *__restrict__ z, long long ldz, const float *__restrict__ a_log, const float *__restrict__ skip,
-                      float *__restrict__ state, T *__restrict__ out, long long ldo, const int *__restrict__ seq_start,
-                      const int *__restrict__ seq_slot, int inner, int N) {
+selective_scan_kernel(const T *x, long long ldx, const float *dt_raw, long long ld_dt,
+                      const float *__restrict__ dt_bias, const float *bc, long long ld_bc, int off_b, int off_c,
+                      const float *z, long long ldz, const float *__restrict__ a_log, const float *__restrict__ skip,
+                      float *state, T *__restrict__ out, long long ldo, const int *seq_start,
+                      const int *seq_slot, int inner, int N) {
   constexpr int CH = SCAN_THREADS / L, NP = L * NS;      // channels of the CTA, padded states
   constexpr int TG = NP <= 64 ? SCAN_GROUP : 8;          // tokens of a group
   constexpr int PAIRS = (TG * CH + SCAN_THREADS - 1) / SCAN_THREADS, ROWS = SCAN_THREADS / CH;   // (token, channel) pairs a thread brings in
@@ -353,11 +353,11 @@ selective_scan_kernel(const T *__restrict__ x, long long ldx, const float *__res
 // values, then B and C at their offsets; w_dt [inner, ldw] in the engine's type.
 template <typename T, int L, int NS>
 __global__ void __launch_bounds__(SS_THREADS)
-selective_step_kernel(const T *__restrict__ x, long long ldx, const float *__restrict__ low, long long ld_low, int low_parts,
+selective_step_kernel(const T *x, long long ldx, const float *low, long long ld_low, int low_parts,
                       long long low_stride, int rank,
                       const T *__restrict__ w_dt, int ldw, const float *__restrict__ dt_bias, int off_b, int off_c,
-                      const float *__restrict__ z, long long ldz, const float *__restrict__ a_log, const float *__restrict__ skip,
-                      float *__restrict__ state, T *__restrict__ out, long long ldo, const int *__restrict__ seq_slot, int inner, int N) {
+                      const float *z, long long ldz, const float *__restrict__ a_log, const float *__restrict__ skip,
+                      float *state, T *__restrict__ out, long long ldo, const int *seq_slot, int inner, int N) {
   constexpr int CH = SS_THREADS / L, NP = L * NS;
   extern __shared__ __align__(16) float low_s[];         // B [NP], C [NP], then the dt input [rank]
   grid_dependents_launch();
@@ -516,7 +516,7 @@ LLM_EXPORT int llm_selective_step(int dtype, const void *x, long long ldx, const
 
 // out [n_rows, cols] bfloat16 = the first n columns of the 32-bit rows `in`, nought beyond them
 __global__ void __launch_bounds__(256)
-rows_cast_kernel(const float *__restrict__ in, long long ld, int n, __nv_bfloat16 *__restrict__ out, int cols, size_t total) {
+rows_cast_kernel(const float *in, long long ld, int n, __nv_bfloat16 *__restrict__ out, int cols, size_t total) {
   grid_dependents_launch();
   grid_dependency_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {

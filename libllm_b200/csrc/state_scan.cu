@@ -203,9 +203,9 @@ __device__ __forceinline__ void scan_group(float2 (&S)[2][ROWS / 2], unsigned re
 
 template <int RULE, int DMAX>
 __global__ void __launch_bounds__(SC_THREADS + 32)
-state_scan_kernel(const float *__restrict__ rec, const float4 *__restrict__ scal, const float *__restrict__ vals, float *__restrict__ state,
-                  float *__restrict__ out, long long ldo, float *__restrict__ den, const int *__restrict__ seq_start,
-                  const int *__restrict__ seq_slot, int n_tokens, int n_heads, int n_kv, int d, int dv, int n_groups_ring, int *status) {
+state_scan_kernel(const float *rec, const float4 *scal, const float *vals, float *state,
+                  float *__restrict__ out, long long ldo, float *__restrict__ den, const int *seq_start,
+                  const int *seq_slot, int n_tokens, int n_heads, int n_kv, int d, int dv, int n_groups_ring, int *status) {
   constexpr int NV = RULE == RULE_BONUS ? 3 : 2;
   constexpr int LANES = scan_lanes(DMAX), ROWS = DMAX / LANES, COLS = 2 * SC_THREADS / LANES;
   extern __shared__ __align__(128) unsigned char sc_smem[];
@@ -432,11 +432,11 @@ struct ConvLane {
 
 template <int CPL, int TAPS, int ROWS>
 __global__ void __launch_bounds__(128, CPL <= 2 && TAPS <= 4 ? 4 : CPL <= 4 && TAPS <= 4 ? 3 : 1)
-delta_pack_kernel(const float *__restrict__ proj, long long ld, int off_b, int off_a, const float *__restrict__ conv, int taps,
-                  float *__restrict__ state, const float *__restrict__ dt_bias, const float *__restrict__ a_log, float key_eps, float q_scale,
-                  float *__restrict__ rec, float4 *__restrict__ scal, float *__restrict__ vals, ValuePlace place, const int *__restrict__ tok_seq,
-                  const int *__restrict__ tok_pos, const int *__restrict__ seq_start, const int *__restrict__ seq_past,
-                  const int *__restrict__ seq_slot, int n_tokens, int n_heads, int n_kv, int d, int dv, int n_chunks) {
+delta_pack_kernel(const float *proj, long long ld, int off_b, int off_a, const float *__restrict__ conv, int taps,
+                  float *state, const float *__restrict__ dt_bias, const float *__restrict__ a_log, float key_eps, float q_scale,
+                  float *__restrict__ rec, float4 *__restrict__ scal, float *__restrict__ vals, ValuePlace place, const int *tok_seq,
+                  const int *tok_pos, const int *seq_start, const int *seq_past,
+                  const int *seq_slot, int n_tokens, int n_heads, int n_kv, int d, int dv, int n_chunks) {
   grid_dependents_launch();
   const int lane = threadIdx.x & 31, item = blockIdx.y * 4 + (threadIdx.x >> 5);
   const bool is_v = item >= n_kv;
@@ -606,8 +606,8 @@ LLM_EXPORT int llm_delta_pack(const float *proj, long long ld, int off_b, int of
 constexpr int BP_WARPS = 4, BP_TT = 4;
 
 __global__ void __launch_bounds__(BP_WARPS * 32)
-bonus_pack_kernel(const float *__restrict__ r, long long ldr, const float *__restrict__ k, long long ldk, const float *__restrict__ v,
-                  long long ldv, const float *__restrict__ x1, long long ldx, int rank, const float *__restrict__ w2,
+bonus_pack_kernel(const float *r, long long ldr, const float *k, long long ldk, const float *v,
+                  long long ldv, const float *x1, long long ldx, int rank, const float *__restrict__ w2,
                   const float *__restrict__ w0, const float *__restrict__ u, int n_tokens, int d, int dv, int w2_shared,
                   float *__restrict__ rec, float4 *__restrict__ scal, float *__restrict__ vals, ValuePlace place) {
   extern __shared__ __align__(16) float bp_sm[];      // tanh(x1) [warps][rank][TT], then W2's rows of the head [d][rank + 1]
@@ -694,9 +694,9 @@ constexpr int MG_TOKENS = 1024, MG_THREADS = 512;
 __device__ __forceinline__ float capped(float x, float cap) { return cap * tanhf(x / cap); }
 
 __global__ void __launch_bounds__(MG_THREADS)
-memory_gates_kernel(const float *__restrict__ proj, long long ld, int off_i, int off_f, const float *__restrict__ bias_i,
-                    const float *__restrict__ bias_f, float cap, float *__restrict__ state_m, float4 *__restrict__ scal,
-                    const int *__restrict__ seq_start, const int *__restrict__ seq_slot, int n_tokens, int n_heads) {
+memory_gates_kernel(const float *proj, long long ld, int off_i, int off_f, const float *__restrict__ bias_i,
+                    const float *__restrict__ bias_f, float cap, float *state_m, float4 *__restrict__ scal,
+                    const int *seq_start, const int *seq_slot, int n_tokens, int n_heads) {
   __shared__ __align__(16) float2 fi[MG_TOKENS];
   __shared__ float m[MG_TOKENS + 1];
   grid_dependents_launch();
@@ -745,7 +745,7 @@ memory_gates_kernel(const float *__restrict__ proj, long long ld, int off_i, int
 constexpr int MP_TT = 4;
 
 __global__ void __launch_bounds__(128)
-memory_pack_kernel(const float *__restrict__ proj, long long ld, int off_q, int off_k, int off_v, float q_scale, float *__restrict__ rec,
+memory_pack_kernel(const float *proj, long long ld, int off_q, int off_k, int off_v, float q_scale, float *__restrict__ rec,
                    float4 *__restrict__ scal, float *__restrict__ vals, ValuePlace place, int n_tokens, int d, int dv) {
   grid_dependents_launch();
   grid_dependency_wait();
@@ -803,8 +803,8 @@ LLM_EXPORT int llm_memory_pack(const float *proj, long long ld, int off_q, int o
 // sigmoid (act 0) or silu (act 1) of 32-bit logits.  LPH lanes to a head, V values of a lane side by side, E times.
 template <typename T, int LPH, int V, int E>
 __global__ void __launch_bounds__(128)
-head_finish_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ den, const float4 *__restrict__ scal,
-                   const float *__restrict__ weight, int shared_weight, const float *__restrict__ gate, long long gate_stride, int act,
+head_finish_kernel(const float *x, long long ldx, const float *den, const float4 *scal,
+                   const float *__restrict__ weight, int shared_weight, const float *gate, long long gate_stride, int act,
                    float eps, float out_scale, int n_tokens, int n_heads, int dv, T *__restrict__ out, long long ldo) {
   grid_dependents_launch();
   const int sub = threadIdx.x % LPH;
@@ -914,9 +914,9 @@ __device__ __forceinline__ void ts_store(T *p, const TsVec<T, V> &r) {
 
 template <typename T, int V, int N_MIX>
 __global__ void __launch_bounds__(TS_THREADS)
-token_shift_kernel(const T *__restrict__ h, long long ldh, const float *__restrict__ mu, T *__restrict__ out, long long mix_stride,
-                   T *__restrict__ state, const int *__restrict__ tok_seq, const int *__restrict__ tok_pos,
-                   const int *__restrict__ seq_start, const int *__restrict__ seq_past, const int *__restrict__ seq_slot, int n_tokens,
+token_shift_kernel(const T *h, long long ldh, const float *__restrict__ mu, T *__restrict__ out, long long mix_stride,
+                   T *state, const int *tok_seq, const int *tok_pos,
+                   const int *seq_start, const int *seq_past, const int *seq_slot, int n_tokens,
                    int width, int n_chunks) {
   grid_dependents_launch();
   const int c = (blockIdx.x * TS_THREADS + threadIdx.x) * V;
@@ -1033,8 +1033,8 @@ __device__ __forceinline__ float step_conv(const StepIn &in, float x, int ch, in
 
 template <int RULE, int DMAX, typename TO>
 __global__ void __launch_bounds__(SS_THREADS)
-state_step_kernel(const StepIn in, float *__restrict__ state, const float *__restrict__ weight, int shared_weight, int act, float eps,
-                  float out_scale, TO *__restrict__ out, long long ldo, const int *__restrict__ seq_slot, int n_heads, int n_kv, int d, int dv) {
+state_step_kernel(const StepIn in, float *state, const float *__restrict__ weight, int shared_weight, int act, float eps,
+                  float out_scale, TO *__restrict__ out, long long ldo, const int *seq_slot, int n_heads, int n_kv, int d, int dv) {
   constexpr int ROWS = DMAX / SS_LANES;
   constexpr int R4 = (ROWS + 3) / 4;                  // 16-byte groups of a lane
   constexpr int NC = R4 <= 2 ? 4 : R4 <= 4 ? 2 : 1;     // columns of a lane whose state is fetched at once
