@@ -278,6 +278,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int row = quarter * 32 + lane;                       // row of the tile = lane of tensor memory
     const unsigned lane_addr = (unsigned)(quarter * 32) << 16;
     const int pos = past + r0 + row;                           // the row's position in its sequence
+    // The last key the row sees.  Rows beyond the sequence, which have a say in when their warp moves its references, see its last
+    // token at most: what lies behind that in the page is an earlier sequence's, and no result is to hang on it.
+    const int vis_hi = min(pos, past + r0 + rows - 1);
     constexpr int HD = 32 * VB;                                // this thread's channels of the output row
     const unsigned o_addr = tmem_o + lane_addr + half * HD;
     float ref = -INFINITY;            // the exponent's reference, already times log2(e) / sqrt(d)
@@ -305,7 +308,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int key = k0 + c * 16 + i;
-              if (!(key <= pos && (key >= vis_lo || key < sink))) own[c][i] = -INFINITY;
+              if (!(key <= vis_hi && (key >= vis_lo || key < sink))) own[c][i] = -INFINITY;
             }
         }
         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, not one of sixteen
@@ -680,6 +683,7 @@ attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q, const _
     const unsigned lane_addr = (unsigned)(quarter * 32) << 16;
     const int pos_lo = past + r0 + x * 128 + quarter * 32;     // the warp's first position
     const int pos = pos_lo + lane;
+    const int vis_hi = min(pos, past + r0 + rows - 1);         // as above: rows beyond the sequence see its last token at most
     const unsigned s_addr = tmem_base + x * FW_BN + lane_addr;
     const unsigned p_addr = tmem_base + S::P_COL + x * S::P_STEP + lane_addr;
     const unsigned o_addr = tmem_base + S::O_COL + x * D + lane_addr;
@@ -711,7 +715,7 @@ attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q, const _
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const int key = k0 + g * 16 + i;
-            if (!(key <= pos && key >= vis_lo)) sc[g][i] = -INFINITY;
+            if (!(key <= vis_hi && key >= vis_lo)) sc[g][i] = -INFINITY;
           }
       }
       float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};

@@ -643,6 +643,34 @@ def test_attention_decode_fused(n_heads, n_kv, d, window, chunk, n_splits):
             close(out[b].view(1, n_heads, d), ref, "bfloat16", scale=max(1.0, float(ref.abs().max())))
 
 
+# last rows that share a warp with rows beyond the sequence (length no multiple of 32), in the first tile and in later ones
+@pytest.mark.parametrize("form", [1, 2])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window,sink", [(None, 0), (100, 3)])
+def test_prompt_attention_does_not_hang_on_old_pages(d, form, window, sink):
+    """A sequence's bits are the same whatever its last page held before, also where the rows that share a warp with its last ones
+    have far larger queries."""
+    from libllm_b200.csrc import ops
+    if form == 2 and sink:
+        pytest.skip("kept first positions are the first form's")
+    page, H, G, lens = 64, 4, 2, [16, 80, 200, 335]
+    for n in lens:
+        K, V, table, _, _ = paged_cache(2, [n, 90], G, d, page, "bfloat16", 171)
+        q = rnd((n + 90, H * d), "bfloat16", 172)
+        q[n:] *= 30
+        start, past = prefill_inputs([n, 90], [n, 90])
+        results = []
+        for factor in (0.0, 30.0):
+            last = int(table[0, (n - 1) // page])
+            K[last, :, (n - 1) % page + 1:] = rnd((G, page - 1 - (n - 1) % page, d), "bfloat16", 174) * factor
+            V[last, :, (n - 1) % page + 1:] = rnd((G, page - 1 - (n - 1) % page, d), "bfloat16", 175) * factor
+            out = torch.empty((n + 90, H * d), dtype=torch.bfloat16, device=DEV)
+            ops.attention_prefill_tc(q, out, K, V, start, past, table, 2, max(n, 90), H, G, d, page, window, 1 / math.sqrt(d), form, sink=sink)
+            ops.check_tc_status()
+            results.append(out[:n].cpu())
+        assert torch.equal(results[0], results[1]), n
+
+
 @pytest.mark.parametrize("n_heads,n_kv,d,window", [(32, 8, 64, None), (3, 1, 64, None), (8, 2, 128, None), (2, 2, 64, 64),
                                                      (6, 3, 128, 130), (4, 1, 64, 37)])
 @pytest.mark.parametrize("form", [1, 2])

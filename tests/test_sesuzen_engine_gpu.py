@@ -112,6 +112,19 @@ def test_unequal_batches_against_each_request_alone(name, dtype):
     assert engine.pages_in_use() == [0] * len(engine.pages_in_use())
 
 
+@pytest.mark.parametrize("name", ["S3", "S6"])
+def test_a_request_is_the_same_behind_any_other(name):
+    """Three requests of unequal prompts in changing order on one engine, each with the same bits every time: nothing is left of the
+    request before, whose pages, slots and states are used again."""
+    engine, c, w = setup(name, "bfloat16", max_tokens=768)
+    requests = [[(f"r{i}{j}", [t * (1 if i else 3) % c["vocab"] for t in S.tokens(c, n + 6, 40 + 3 * i + j)], n) for j, n in enumerate((208, 67, 145))] for i in range(3)]
+    first = {}
+    for k in range(60):
+        i = k * k % 3 if k % 5 else 2
+        for rid, rows in replay_batch(engine, requests[i]).items():
+            assert torch.equal(first.setdefault(rid, rows), rows), f"{rid}, pass {k}"
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", ["S2", "S3", "S4", "S6"])
 def test_long_decoding(name, dtype):
