@@ -581,16 +581,14 @@ gated_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       const int f = ((tile / tok_tiles) * 2 + (int)rank) * GP_FEATURES + quarter * 16 + (lane & 15);
       const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * GP_TOKENS + half * (GP_TOKENS / 2));
       float even[16], odd[16];
-      tc_ld16_issue(taddr, even);
 #pragma unroll 1
-      for (int c = 0; c < CHUNKS; c += 2) {
+      for (int c = 0; c < CHUNKS; c += 2) {          // two loads on their way, none from one round to the next
+        tc_ld16_issue(taddr + c * 16, even);
+        tc_ld16_issue(taddr + (c + 1) * 16, odd);
         tc_ld_wait();
         tc_ld_ready(even);
-        tc_ld16_issue(taddr + (c + 1) * 16, odd);
-        store_turns(even, out, ldo, f, n_out, tok0 + c * 16, M, glu);
-        tc_ld_wait();
         tc_ld_ready(odd);
-        if (c + 2 < CHUNKS) tc_ld16_issue(taddr + (c + 2) * 16, even);
+        store_turns(even, out, ldo, f, n_out, tok0 + c * 16, M, glu);
         store_turns(odd, out, ldo, f, n_out, tok0 + (c + 1) * 16, M, glu);
       }
       tc_fence_before();

@@ -90,3 +90,25 @@ def test_no_load_may_leave_the_wait_behind(file):
         if kernel and re.search(r"__ldg\s*\(", body):
             wrong.append(f"{name}: __ldg")
     assert not wrong, "\n".join(wrong)
+
+
+def test_loads_from_tensor_memory_are_waited_for_where_they_are_issued():
+    """What `tcgen05.ld` writes is undefined until the wait: between the two a register may not even be copied, which a compiler does where
+    the load's block ends (a loop's back edge, an if).  So the wait follows in the same block, and a load with its wait is one statement."""
+    text = open(os.path.join(CSRC, "tc_common.cuh")).read()
+    one = text[text.index("void tc_ld16(unsigned"):]
+    assert re.search(r"asm volatile\([^;]*tcgen05\.ld[^)]*?tcgen05\.wait::ld", one[:one.index("\n}\n")], re.S)
+    loads = 0
+    for file, name, _, body, _ in KERNELS:
+        for m in re.finditer(r"tc_ld16_issue\(", body):
+            if name == "tc_ld16_issue":
+                continue
+            loads += 1
+            line = body[body.rfind("\n", 0, m.start()) + 1:m.start()]
+            assert not re.search(r"\bif\b", line), f"{file}: {name}: a load that is issued or not"
+            at, depth = m.end(), 0
+            while not body.startswith("tc_ld_wait()", at):
+                depth += {"{": 1, "}": -1}.get(body[at], 0)
+                assert depth >= 0, f"{file}: {name}: the block ends before the wait"
+                at += 1
+    assert loads >= 10
