@@ -191,9 +191,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       unsigned phase = 0;
       bool ok = true;
       for (int j = 0; j < n_tiles && ok; ++j) {
+        const int row = (pt[tile_of(j)] * n_kv + kvh) * FT_BN;      // looked up while the stage is waited for
         ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, 11));
         if (!ok) break;
-        const int row = (pt[tile_of(j)] * n_kv + kvh) * FT_BN;
         const unsigned tk = smem_u32(sKV + (size_t)stage * S::KV_BYTES), tv = tk + S::K_BYTES;
         if (leader) {
           mbar_expect_tx(bar_full + 8 * stage, S::KV_BYTES);
@@ -565,12 +565,12 @@ attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q, const _
       unsigned phase = 0;
       bool ok = true;
       for (int j = 0; j < n_tiles && ok; ++j) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, 31));
-        if (!ok) break;
         // A tile's second page may lie behind the sequence's end: the first is loaded in its place
         // (finite numbers, all masked).
         const int p0 = 2 * (first_tile + j), p1 = min(p0 + 1, last_page);
         const int row0 = (pt[p0] * n_kv + kvh) * 64, row1 = (pt[p1] * n_kv + kvh) * 64;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, 31));
+        if (!ok) break;
         const unsigned dk = smem_u32(sKV + (size_t)stage * 2 * S::KV_BYTES), dv = dk + S::KV_BYTES;
         if (leader) {
           mbar_expect_tx(bar_full + 8 * stage, 2 * S::KV_BYTES);

@@ -179,9 +179,9 @@ sigmoid_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       unsigned phase = 0;
       bool ok = true;
       for (int j = 0; j < n_tiles && ok; ++j) {
+        const int row = (pt[first_tile + j] * n_kv + kvh) * SA_BN;   // looked up while the stage is waited for
         ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, 51));
         if (!ok) break;
-        const int row = (pt[first_tile + j] * n_kv + kvh) * SA_BN;
         const unsigned dk = smem_u32(sKV + (size_t)stage * S::KV_BYTES), dvv = dk + S::K_BYTES;
         if (leader) {
           mbar_expect_tx(bar_full + 8 * stage, S::KV_BYTES);
