@@ -124,9 +124,10 @@ attention_generic_kernel(const T *q, long long q_stride, T *__restrict__ out,
         if (sig.cap > 0.f) s = sig.cap * tanhf(s / sig.cap);
         pj = valid ? 1.f / (1.f + expf(-(s + bias))) : 0.f;
       } else {
-        const float m_new = fmaxf(m, warp_max(s));          // finite: lane 0 always holds a key
-        pj = valid ? expf(s - m_new) : 0.f;
-        const float alpha = expf(m - m_new);                // 0 on the first block (m = -inf)
+        // minus infinity while this warp has met no other score (a product that overflows): such keys weigh nothing, they are not NaN
+        const float m_new = fmaxf(m, warp_max(s)), ref = m_new == -INFINITY ? 0.f : m_new;
+        pj = valid ? expf(s - ref) : 0.f;
+        const float alpha = expf(m - ref);                  // 0 on the first block (m = -inf)
         l = l * alpha + warp_sum(pj);
 #pragma unroll
         for (int i = 0; i < NI; ++i) acc[i] *= alpha;

@@ -166,6 +166,25 @@ def test_attention_finds_one_far_key_among_hundreds(dtype):
     assert float((out.float().cpu()[0] - vs[0][3, 0].float()).abs().max()) < 0.2
 
 
+# blocks of 32 keys of the first, a later and several warps; all but the last key
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("lo,hi", [(0, 32), (32, 64), (32, 160), (0, 199)])
+def test_keys_of_score_minus_infinity_weigh_nothing(dtype, lo, hi):
+    from libllm_b200.csrc import ops
+    d, page, L = 64, 64, 200
+    K, V, table, ks, vs = paged_cache(1, [L], 1, d, page, dtype, 18)
+    q = rnd((1, d), dtype, 19)
+    q[0, 0] = 1.0
+    for j in range(lo, hi):
+        K[int(table[0, j // page]), 0, j % page, 0] = float("-inf")
+    out = torch.empty((1, d), dtype=DT[dtype], device=DEV)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ops.attention_generic(q, out, K, V, torch.zeros(1, **i32), torch.tensor([L - 1], **i32), table, 1, 1, d, page, None, 1 / math.sqrt(d))
+    seen = [j for j in range(L) if not lo <= j < hi]
+    ref = P.attention_scores_softmax_values(q.cpu().view(1, 1, d), ks[0][seen], vs[0][seen])
+    close(out.view(1, 1, d), ref, dtype, scale=max(1.0, float(ref.abs().max())))
+
+
 @pytest.mark.parametrize("dtype,in_dtype", [("float32", "float32"), ("bfloat16", "bfloat16"), ("bfloat16", "float32")])
 @pytest.mark.parametrize("n_heads,n_kv,d", [(4, 2, 16), (3, 1, 96)])
 def test_rope_and_cache_write(dtype, in_dtype, n_heads, n_kv, d):
