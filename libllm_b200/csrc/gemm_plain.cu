@@ -258,10 +258,14 @@ static int launch_tile(const float *A, long long lda, const float *W, long long 
                        int K, cudaStream_t stream) {
   using S = TileShape;
   LLM_CHECK_CUDA(llm_allow_smem(gemm_tile_kernel, S::SMEM), "gemm_plain attribute");
-  const int rows = (M + S::RM - 1) / S::RM;
-  LLM_REQUIRE(rows <= 65535, "gemm_plain: %d rows are too many for one launch", M);
-  LLM_CHECK_CUDA(llm_launch(gemm_tile_kernel, dim3((N + 63) / 64, rows), dim3(256), S::SMEM, stream, A, lda, W, ldw, bias, C, ldc, M, N, K),
-                 "gemm_plain launch");
+  LLM_REQUIRE(M <= 65535 * BM, "gemm_plain: %d rows are too many", M);        // as for the tiles of 64 rows below
+  constexpr int MOST = 65535 * S::RM;          // rows of one launch
+  for (long long m0 = 0; m0 < M; m0 += MOST) {
+    const int m = (int)(M - m0 < MOST ? M - m0 : MOST);
+    LLM_CHECK_CUDA(llm_launch(gemm_tile_kernel, dim3((N + 63) / 64, (m + S::RM - 1) / S::RM), dim3(256), S::SMEM, stream, A + m0 * lda, lda, W, ldw,
+                              bias, C + m0 * ldc, ldc, m, N, K),
+                   "gemm_plain launch");
+  }
   return LLM_OK;
 }
 // Both kernels give a row the same bits, so the choice may look at everything.  Eight rows on the kernel for few cost 59 us at a W of

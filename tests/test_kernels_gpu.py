@@ -558,6 +558,16 @@ def test_norm_of_prompt_rows_has_the_bits_of_a_row_alone(hidden, parts, scaled):
     assert bool(((got.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all())
 
 
+def test_32_bit_product_of_more_rows_than_one_launch_takes():
+    from libllm_b200.csrc import ops
+    M = 65535 * 32 + 40
+    x, w = rnd((M, 4), "float32", 64), rnd((3, 4), "float32", 65)
+    out = torch.full((M, 3), float("nan"), device=DEV)
+    ops.gemm_plain(x, w, out)
+    ref = x.double() @ w.double().T
+    assert float((out.double() - ref).abs().max()) < 8 * 2 ** -24 * float((x.double().abs() @ w.double().abs().T).max())     # 4 products, 8 roundings at most
+
+
 # one part with work and eight, parts that end inside a block, widths beside the tiles; 4-byte rows take the general kernel
 @pytest.mark.parametrize("K,N", [(4, 1), (36, 15), (252, 16), (260, 17), (1028, 130), (2048, 64), (97, 33)])
 def test_32_bit_product_rows_do_not_depend_on_the_batch(K, N):
