@@ -202,16 +202,19 @@ static int launch_generic(int dtype, const void *q, long long q_stride, void *ou
   LLM_REQUIRE(sink == 0 || block == 0, "attention: kept first positions go with a window, not with a block mask");
   // 16-byte loads of key rows where rows start on such a boundary
   const int vec = (dtype == LLM_F32 ? d % 4 == 0 : d % 8 == 0) && (uintptr_t)kcache % 16 == 0;
-  const long long blocks = (long long)n_tokens * n_heads;
-  LLM_REQUIRE(blocks < 2147483647LL, "attention: too many tokens for one launch");
+  // a CTA to a (token, head): launches of as many tokens as a grid has room for
+  const int tokens = n_tokens < 2147483647LL / n_heads ? n_tokens : (int)(2147483647LL / n_heads);
+  LLM_REQUIRE(((long long)n_tokens * n_heads + WARPS - 1) / WARPS < 2147483647LL, "attention: too many tokens");
   const int widest = d > dv ? d : dv;
   const SigmoidWeights sw = sig ? *sig : SigmoidWeights{};
 #define GENERIC_RUN(T, MAXD, SIG)                                                                                        \
-  LLM_CHECK_CUDA(llm_launch(attention_generic_kernel<T, MAXD, SIG>, dim3((unsigned)blocks), dim3(WARPS * 32), 0, stream,      \
-                            (const T *)q, q_stride, (T *)out, out_stride, (const T *)kcache, (const T *)vcache, tok_seq, tok_pos, page_table,  \
-                            pt_stride, n_heads, n_kv, d, dv, page_size, window, block, sink, scale, gate, gate_stride, vec, v_ld,     \
-                            null_score, null_scores, sw),                                                                \
-                 "attention_generic")
+  for (long long t0 = 0; t0 < n_tokens; t0 += tokens)                                                                     \
+    LLM_CHECK_CUDA(llm_launch(attention_generic_kernel<T, MAXD, SIG>, dim3((unsigned)((n_tokens - t0 < tokens ? n_tokens - t0 : tokens) * n_heads)), \
+                              dim3(WARPS * 32), 0, stream, (const T *)q + t0 * q_stride, q_stride, (T *)out + t0 * out_stride, out_stride,     \
+                              (const T *)kcache, (const T *)vcache, tok_seq + t0, tok_pos + t0, page_table, pt_stride, n_heads, n_kv, d, dv,  \
+                              page_size, window, block, sink, scale, gate ? gate + t0 * gate_stride : gate, gate_stride, vec, v_ld, null_score, \
+                              null_scores, sw),                                                                           \
+                   "attention_generic")
 #define GENERIC_GO(T, MAXD)                                                                                              \
   do {                                                                                                                   \
     if (sig) GENERIC_RUN(T, MAXD, true);                                                                                 \

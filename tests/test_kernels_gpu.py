@@ -166,6 +166,20 @@ def test_attention_finds_one_far_key_among_hundreds(dtype):
     assert float((out.float().cpu()[0] - vs[0][3, 0].float()).abs().max()) < 0.2
 
 
+def test_attention_of_more_heads_and_tokens_than_one_grid_takes():
+    """One key each, so that every result is its value; 2^31 + 1,024 (token, head) pairs."""
+    from libllm_b200.csrc import ops
+    T, H = 2 ** 21 + 1, 1024
+    i32 = dict(dtype=torch.int32, device=DEV)
+    K, V = (torch.full((1, 1, 16, 1), x, dtype=torch.bfloat16, device=DEV) for x in (1.0, 0.75))
+    q = torch.zeros((T, H), dtype=torch.bfloat16, device=DEV)
+    out = torch.zeros_like(q)
+    ops.attention_generic(q, out, K, V, torch.zeros(T, **i32), torch.zeros(T, **i32), torch.zeros((1, 1), **i32), H, 1, 1, 16, None, 1.0)
+    assert float(out.min()) == float(out.max()) == 0.75
+    del q, out
+    torch.cuda.empty_cache()
+
+
 # blocks of 32 keys of the first, a later and several warps; all but the last key
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("lo,hi", [(0, 32), (32, 64), (32, 160), (0, 199)])
