@@ -606,7 +606,8 @@ def test_32_bit_product_rows_do_not_depend_on_the_batch(K, N):
 # widths of whole groups of 16 (gate and up rows in turns) and others; rows at the tiles' edges
 @pytest.mark.parametrize("M,I,K", [(1, 64, 64), (5, 173, 80), (8, 8192, 2048), (40, 300, 256), (200, 128, 136), (257, 391, 200),
                                    (1000, 1024, 512), (1, 16, 8), (16, 48, 136), (17, 80, 72), (33, 208, 200), (64, 1040, 64), (65, 48, 64),
-                                   (512, 4752, 8), (640, 3216, 72), (1025, 1904, 200)])        # two SMs to a tile, ragged on both sides
+                                   (512, 4752, 8), (640, 3216, 72), (1025, 1904, 200),        # two SMs to a tile, ragged on both sides
+                                   (2000, 5136, 456), (1280, 8208, 1096)])      # ... every pair's ring and both accumulators used again
 def test_tensor_core_product_with_swiglu(M, I, K):
     from libllm_b200.csrc import ops
     x = rnd((M, K), "bfloat16", 54)

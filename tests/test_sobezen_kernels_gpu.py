@@ -222,6 +222,47 @@ def test_latent_tokens_behind_cached_rows_are_the_same_alone_and_together():
         assert torch.equal(results[0][i][0], results[1][i][0]), f"latent layer {i}"
 
 
+# runs at and beyond the eight whose values a thread of the join asks for together, some without keys; widths that leave threads idle and that
+# take them all, output rows on 8 bytes and not
+@pytest.mark.parametrize("R,rot,heads,row_gap", [(64, 16, 5, 0), (512, 32, 3, 2), (512, 64, 2, 0), (96, 8, 33, 4)])
+@pytest.mark.parametrize("n_splits", [1, 7, 8, 9, 17, 40])
+def test_latent_runs_are_joined(n_splits, R, rot, heads, row_gap):
+    """All heads of two tokens over the cached rows, against the softmax in 64 bits; probabilities are rounded to bfloat16 in the kernel."""
+    from ctypes import c_float, c_int, c_longlong, c_void_p
+    from libllm_b200.csrc import ops
+    g = torch.Generator().manual_seed(R + n_splits)
+    lens, row = [1290, 700], R + rot
+    pages = [(n + PAGE - 1) // PAGE for n in lens]
+    order = torch.randperm(sum(pages), generator=g)
+    table = torch.zeros(2, max(pages), dtype=torch.int32)
+    cache = torch.zeros(sum(pages), PAGE, row)
+    data, at = [], 0
+    for b, n in enumerate(lens):
+        rows = bf(torch.randn(n, row, generator=g))
+        data.append(rows.double())
+        for j in range(pages[b]):
+            table[b, j] = order[at]
+            part = rows[j * PAGE:(j + 1) * PAGE]
+            cache[order[at], :len(part)] = part
+            at += 1
+    q = bf(torch.randn(2, heads * row, generator=g))
+    out = torch.zeros(2, heads * R + row_gap, dtype=torch.bfloat16, device=DEV)
+    ws = torch.full((2 * heads * n_splits * (R + 2),), float("nan"), device=DEV)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    qd, cd, td, seq, pos = q.to(torch.bfloat16).to(DEV), cache.to(torch.bfloat16).to(DEV), table.to(DEV), torch.arange(2, **i32), torch.tensor(lens, **i32) - 1
+    scale = 2.0 / row ** 0.5
+    ops._call("latent_tc", "llm_latent_decode", [c_void_p, c_longlong, c_void_p, c_int] + [c_void_p] * 3 + [c_int] * 6 + [c_float, c_void_p, c_longlong,
+              c_void_p, c_int, c_void_p], qd.data_ptr(), qd.stride(0), cd.data_ptr(), PAGE, seq.data_ptr(), pos.data_ptr(), td.data_ptr(), td.stride(0),
+              2, heads, R, rot, n_splits, scale, out.data_ptr(), out.stride(0), ws.data_ptr(), 0, torch.cuda.current_stream().cuda_stream)
+    for b in range(2):
+        p = torch.softmax(q[b].double().view(heads, row) @ data[b].T * scale, -1)
+        want, size = p @ data[b][:, :R], p @ data[b][:, :R].abs()
+        got = out[b, :heads * R].double().cpu().view(heads, R)
+        # a probability's rounding (2^-9) and the result's, of the terms' sizes; 32-bit sums and exponentials beside them are nothing
+        assert bool(((got - want).abs() <= 2.2 * 2 ** -9 * (size + want.abs()) + 1e-6).all())
+    assert float(out[:, heads * R:].abs().max() if row_gap else 0.0) == 0.0
+
+
 # tokens at which another instantiation takes over, heads of one and of several fetches of w_uk, latents with an odd width
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,H,d,rot,R,dv", [(1, 2, 6, 2, 22, 10), (2, 3, 64, 32, 512, 64), (3, 1, 65, 0, 33, 7), (4, 2, 80, 4, 520, 9),
