@@ -17,11 +17,13 @@
 // 90 KB (few tokens) to 200 KB (prompts) of loads are in flight per SM, which is what a stream from
 // HBM needs.
 //
-// SwiGLU, or any gated unit of GluShape: W is the stacked gate|up matrix [2I, K].  A tile holds gate rows f..f+63 in its lanes
-// 0-63 and up rows I+f..I+f+63 in lanes 64-127; the epilogue warps of the upper half hand their
-// values over through shared memory and the lower half stores silu(gate) * up: the stacked
-// product never reaches memory (the reference runs a separate launch, src/flint/cuda/swiglu.cu:29-59,
-// after cuBLAS, src/flint/cuda/gemm_cublas.cc:160-197).
+// SwiGLU, or any gated unit of GluShape: W is the stacked gate|up matrix [2I, K], and the stacked product never reaches memory (the
+// reference runs a separate launch, src/flint/cuda/swiglu.cu:29-59, after cuBLAS, src/flint/cuda/gemm_cublas.cc:160-197).  Which form
+// a launch takes (dispatch_tc):
+//   up to 64 tokens      a tile of 64 features, gate and up rows in turns of 16, traded by shuffles within an epilogue warp; where I is
+//                        no multiple of 16, gate rows in lanes 0-63 and up rows in lanes 64-127, handed over through shared memory;
+//   prompts, takes_pair  two SMs to a tile (gated_pair_kernel, below), rows in turns as above;
+//   other prompts        a tile of 128 gate rows and one of 128 up rows with an accumulator each.
 //
 // Rows of W, tokens and K beyond the matrices are zero-filled by TMA and never stored, so every
 // size is taken (K a multiple of 8: rows must start on 16 bytes).  Every wait on a barrier has a

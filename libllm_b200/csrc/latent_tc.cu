@@ -600,8 +600,8 @@ latent_join_kernel(const float *ws_o, const float *ws_ml, int n_splits, int kv_r
   const int h = blockIdx.x, tok = blockIdx.y;
   const float *ml = ws_ml + ((size_t)tok * n_heads + h) * n_splits * 2;
   const float *po = ws_o + ((size_t)tok * n_heads + h) * n_splits * (size_t)kv_rank;
-  // four channels to a thread, its first runs' values asked for together with the maxima and sums: eight runs' join 7.4 us, now
-  // 4.6 for sixteen
+  // four channels to a thread, its first runs' values asked for together with the maxima and sums: 4.6 us for sixteen runs, 7.4 for eight
+  // when a thread asked for them channel by channel behind the weights
   constexpr int AHEAD = 8;
   const bool quads = kv_rank % 4 == 0 && ldo % 4 == 0 && (uintptr_t)out % 8 == 0 && (uintptr_t)ws_o % 16 == 0;
   float4 v[AHEAD];

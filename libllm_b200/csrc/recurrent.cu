@@ -205,9 +205,9 @@ LLM_EXPORT int llm_causal_conv(int dtype, const void *h, long long ldh, void *ou
 //   decay   w = exp(-decay_scale * sigmoid(w0 + W2 tanh(x1)))       x1 = the low-rank projection
 //   unit    u = k / sqrt(sum(k^2) + key_eps)
 //   removal b = sigmoid(a + a_bias) * u
-// prep [tokens, heads, 3, d]: w, b, u.  A CTA takes one head and a run of tokens, a warp one token
-// at a time: the head's rows of W2 ([d, rank], each row padded by one value so that the lanes'
-// reads fall on different banks) lie in shared memory when they fit, tanh(x1) is taken once per
+// prep [tokens, heads, 3, d]: w, b, u.  A CTA takes one head and a run of tokens, a warp four tokens
+// at a time (one where a decay input is too wide for four): the head's rows of W2 ([d, rank], each row padded by one value so that the
+// lanes' reads fall on different banks) lie in shared memory when they fit, tanh(x1) is taken once per
 // token and warp.  Sums over the head run in lane order then the shuffle tree, whatever the launch.
 constexpr int DP_WARPS = 4;
 constexpr int DP_TOKENS = 32;                        // tokens of a CTA
