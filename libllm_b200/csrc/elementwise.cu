@@ -405,14 +405,14 @@ static int launch_add_rmsnorm(float *resid, const void *delta, int n_parts, size
                        (uintptr_t)col_scale % 16 == 0 && (uintptr_t)col_bias % 16 == 0;
   if (aligned && hidden <= 4 * VPT * THREADS && n_parts <= 16) {
     // A warp to a row from as many rows as give every SM its warps (below, a row's own loads want a block's
-    // threads), where a lane holds the row: up to 4,096 columns, 2,048 with something to add (two
-    // rows' worth of registers).
-    if (n_rows >= 1024 && !rows && out && n_parts <= 1 && hidden > 512 && hidden <= (n_parts ? 2048 : 4096)) {
+    // threads), where a lane holds the row: up to 4,096 columns, 1,024 with something to add (two rows' worth of registers: 8,192 rows
+    // of 1,024 32.7 -> 24.6 us, but with 2,048 columns 164 registers leave 12 warps an SM: 2,048 rows 16.4 -> 18.4, 8,192 rows 43.0 either way).
+    if (n_rows >= 1024 && !rows && out && n_parts <= 1 && hidden > 512 && hidden <= (n_parts ? 1024 : 4096)) {
 #define NORM_ROWS(V_, D_)                                                                                                 \
   llm_launch(norm_rows_kernel<TD, TO, V_, D_>, (n_rows + 3) / 4, 128, 0, stream, resid, (const TD *)delta, weight, eps, (TO *)out, n_rows, \
              hidden, col_scale, col_bias)
       if (hidden <= 1024) n_parts ? NORM_ROWS(8, true) : NORM_ROWS(8, false);
-      else if (hidden <= 2048) n_parts ? NORM_ROWS(16, true) : NORM_ROWS(16, false);
+      else if (hidden <= 2048) NORM_ROWS(16, false);
       else if (hidden <= 3072) NORM_ROWS(24, false);
       else NORM_ROWS(32, false);
 #undef NORM_ROWS
