@@ -297,12 +297,14 @@ delta_prepare_kernel(const float *proj, long long ld, int off_k, int off_a, int 
 // each with d / LANES of its rows in registers, own column j for the whole step and walk the
 // sequence's tokens in order.  The tokens' vectors (w, b, u from the preparation, k and r from the
 // product's rows, the CTA's columns of v) come through a ring of 8 or 16 tokens in shared memory,
-// filled by a third warp's asynchronous copies that run that many tokens ahead of the arithmetic (what a token
+// filled by a fifth warp's asynchronous copies that run that many tokens ahead of the arithmetic (what a token
 // needs was written by the kernels just before and may come from DRAM), so that a token costs its arithmetic and a
 // share of a barrier, not a trip to memory.  (Issued by the warps of the recurrence themselves, the copies and their
-// address arithmetic cost a scan of 2,048 tokens 0.3 ms of its 0.86.)  Sums run over four partial sums in
+// address arithmetic cost a scan of 2,048 tokens 0.3 ms of its 0.86.)  Four warps of a CTA, so that each has an SM sub-partition of its
+// own, and rows in pairs: 2,000 and 841 tokens of 32 heads of 64 take 536 -> 482 us; what is left is a warp's chain (a read of shared
+// memory, four multiplications, two shuffles, one multiplication a token) and the barriers.  Sums run over four partial sums in
 // a fixed order, then the lanes' shuffle tree.  state[slot][head][j][i] (a column's rows together).
-constexpr int DR_THREADS = 64;
+constexpr int DR_THREADS = 128;
 constexpr int DR_STAGES_MAX = 16;                   // tokens of the ring: 16 where they fit 48 KB of shared memory, else 8
 
 __device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
@@ -315,54 +317,88 @@ __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// One token of one column: this thread's share S[ROWS] of the column, the token's vectors w, b, u, k, r (each
-// VLEN floats on; `vecs` points at this thread's share of w, 16-byte aligned), the column's value v.  Returns the
-// column's read-out S^T r, summed over the LANES lanes of the column.  Sums run over four partial sums in a
-// fixed order, then the lanes' shuffle tree: the same wherever a token is computed.
-template <int ROWS, int LANES>
-__device__ __forceinline__ float delta_token(float (&S)[ROWS], const float *vecs, int VLEN, float v) {
-  const float4 *w4 = reinterpret_cast<const float4 *>(vecs), *b4 = reinterpret_cast<const float4 *>(vecs + VLEN);
-  const float4 *u4 = reinterpret_cast<const float4 *>(vecs + 2 * VLEN), *k4 = reinterpret_cast<const float4 *>(vecs + 3 * VLEN);
-  const float4 *r4 = reinterpret_cast<const float4 *>(vecs + 4 * VLEN);
-  float p4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < ROWS / 4; ++i) {
-    const float4 uu = u4[i];
-    p4[0] = fmaf(uu.x, S[4 * i], p4[0]);
-    p4[1] = fmaf(uu.y, S[4 * i + 1], p4[1]);
-    p4[2] = fmaf(uu.z, S[4 * i + 2], p4[2]);
-    p4[3] = fmaf(uu.w, S[4 * i + 3], p4[3]);
-  }
-  float us = (p4[0] + p4[1]) + (p4[2] + p4[3]);
-  // what does not wait for u^T S is taken while its shuffles are on their way: e = w S + k v, then S = e - b (u^T S)
-  float e[ROWS];
-#pragma unroll
-  for (int i = 0; i < ROWS / 4; ++i) {
-    const float4 ww = w4[i], kk = k4[i];
-    e[4 * i] = fmaf(ww.x, S[4 * i], kk.x * v);
-    e[4 * i + 1] = fmaf(ww.y, S[4 * i + 1], kk.y * v);
-    e[4 * i + 2] = fmaf(ww.z, S[4 * i + 2], kk.z * v);
-    e[4 * i + 3] = fmaf(ww.w, S[4 * i + 3], kk.w * v);
-  }
-#pragma unroll
-  for (int o = 1; o < LANES; o <<= 1) us += __shfl_xor_sync(0xffffffffu, us, o);
-  float a4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < ROWS / 4; ++i) {
-    const float4 bq = b4[i], rr = r4[i];
-    S[4 * i] = fmaf(-bq.x, us, e[4 * i]);
-    S[4 * i + 1] = fmaf(-bq.y, us, e[4 * i + 1]);
-    S[4 * i + 2] = fmaf(-bq.z, us, e[4 * i + 2]);
-    S[4 * i + 3] = fmaf(-bq.w, us, e[4 * i + 3]);
-    a4[0] = fmaf(S[4 * i], rr.x, a4[0]);
-    a4[1] = fmaf(S[4 * i + 1], rr.y, a4[1]);
-    a4[2] = fmaf(S[4 * i + 2], rr.z, a4[2]);
-    a4[3] = fmaf(S[4 * i + 3], rr.w, a4[3]);
-  }
-  float acc = (a4[0] + a4[1]) + (a4[2] + a4[3]);
+// Two neighbouring rows of a column in one register pair: the packed forms round each half as the single ones do and take half
+// the issue slots.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) { return (f32x2)__float_as_uint(hi) << 32 | __float_as_uint(lo); }
+__device__ __forceinline__ float pair_sum(f32x2 p) { return __uint_as_float((unsigned)p) + __uint_as_float((unsigned)(p >> 32)); }
+__device__ __forceinline__ f32x2 fma_pair(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul_pair(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// One token of one column: this thread's share S of the column (ROWS rows in pairs), the token's vectors w, b, u, k, r (each
+// VLEN floats on; `vecs` points at this thread's share of w, 16-byte aligned), the column's value v.  Returns this
+// thread's share of the column's read-out S^T r, which delta_sum adds over the LANES lanes of the column.  Sums run over four
+// partial sums in a fixed order, then the lanes' shuffle tree: the same wherever a token is computed.  `before`: the share of the
+// token before, which is added over the lanes here, its shuffles beside those that this token waits for.
+template <int LANES>
+__device__ __forceinline__ float delta_sum(float acc) {
 #pragma unroll
   for (int o = 1; o < LANES; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   return acc;
+}
+template <int ROWS, int LANES>
+__device__ __forceinline__ float delta_token(f32x2 (&S)[ROWS / 2], const float *vecs, int VLEN, float v, float &before) {
+  const ulonglong2 *w4 = reinterpret_cast<const ulonglong2 *>(vecs), *b4 = reinterpret_cast<const ulonglong2 *>(vecs + VLEN);
+  const ulonglong2 *u4 = reinterpret_cast<const ulonglong2 *>(vecs + 2 * VLEN), *k4 = reinterpret_cast<const ulonglong2 *>(vecs + 3 * VLEN);
+  const ulonglong2 *r4 = reinterpret_cast<const ulonglong2 *>(vecs + 4 * VLEN);
+  f32x2 p01 = 0, p23 = 0;
+#pragma unroll
+  for (int i = 0; i < ROWS / 4; ++i) {
+    const ulonglong2 uu = u4[i];
+    p01 = fma_pair(uu.x, S[2 * i], p01);
+    p23 = fma_pair(uu.y, S[2 * i + 1], p23);
+  }
+  float us = pair_sum(p01) + pair_sum(p23);
+  // what does not wait for u^T S is taken while its shuffles are on their way: e = w S + k v, then S = e - b (u^T S)
+  const f32x2 vv = pair_of(v, v);
+  f32x2 e[ROWS / 2];
+#pragma unroll
+  for (int i = 0; i < ROWS / 4; ++i) {
+    const ulonglong2 ww = w4[i], kk = k4[i];
+    e[2 * i] = fma_pair(ww.x, S[2 * i], mul_pair(kk.x, vv));
+    e[2 * i + 1] = fma_pair(ww.y, S[2 * i + 1], mul_pair(kk.y, vv));
+  }
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) {
+    us += __shfl_xor_sync(0xffffffffu, us, o);
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+  }
+  const f32x2 cut = pair_of(-us, -us);
+  f32x2 a01 = 0, a23 = 0;
+#pragma unroll
+  for (int i = 0; i < ROWS / 4; ++i) {
+    const ulonglong2 bq = b4[i], rr = r4[i];
+    S[2 * i] = fma_pair(bq.x, cut, e[2 * i]);
+    S[2 * i + 1] = fma_pair(bq.y, cut, e[2 * i + 1]);
+    a01 = fma_pair(S[2 * i], rr.x, a01);
+    a23 = fma_pair(S[2 * i + 1], rr.y, a23);
+  }
+  return pair_sum(a01) + pair_sum(a23);
+}
+// A thread's share of a column of the state in memory (rows of its own from `first` on, those from d on are zero).
+template <int ROWS>
+__device__ __forceinline__ void delta_load_state(f32x2 (&S)[ROWS / 2], const float *sp, int first, int d, bool live) {
+#pragma unroll
+  for (int i = 0; i < ROWS / 2; ++i) {
+    const float lo = live && first + 2 * i < d ? sp[2 * i] : 0.f, hi = live && first + 2 * i + 1 < d ? sp[2 * i + 1] : 0.f;
+    S[i] = pair_of(lo, hi);
+  }
+}
+template <int ROWS>
+__device__ __forceinline__ void delta_store_state(const f32x2 (&S)[ROWS / 2], float *sp, int first, int d) {
+#pragma unroll
+  for (int i = 0; i < ROWS / 2; ++i) {
+    if (first + 2 * i < d) sp[2 * i] = __uint_as_float((unsigned)S[i]);
+    if (first + 2 * i + 1 < d) sp[2 * i + 1] = __uint_as_float((unsigned)(S[i] >> 32));
+  }
 }
 
 template <int DMAX, int LANES, bool VEC>
@@ -396,36 +432,40 @@ delta_rule_kernel(const float *proj, long long ld, int off_r, int off_k, int off
 
   if (tid >= DR_THREADS) {
     // ------------------------------------------------------------ the loader warp
-    // Its lanes' copies of a token, worked out once: where from (an offset into the token's prepared vectors, or into
-    // its row of the product, marked by bit 30) and where to (element i of a vector lies at (i / ROWS) * PAD + i % ROWS).
+    // Its lanes' copies of a token, worked out once: where from (the token's prepared vectors, or its row of the product) and where
+    // to (element i of a vector lies at (i / ROWS) * PAD + i % ROWS).
     const int lane = tid - DR_THREADS;
-    int from[PER], to[PER];
+    const float *from[PER];
+    int to[PER];
+    long long next[PER];                              // from one token's to the next one's
     const int per_vec = d / UNIT, n_v = (min(COLS, dv - j0) + UNIT - 1) / UNIT;
+    const float *row = proj + (size_t)start * ld, *pr = prep + ((size_t)start * n_heads + hd) * 3 * d;
 #pragma unroll
     for (int e = 0; e < PER; ++e) {
       const int idx = lane + e * 32;
-      from[e] = to[e] = -1;
+      from[e] = row;
+      next[e] = ld;
+      to[e] = -1;
       if (idx < 5 * per_vec) {
         const int which = idx / per_vec, i = (idx - which * per_vec) * UNIT;
-        from[e] = which < 3 ? which * d + i : ((which == 3 ? off_k : off_r) + hd * d + i) | (1 << 30);
+        from[e] = which < 3 ? pr + which * d + i : row + (which == 3 ? off_k : off_r) + hd * d + i;
+        if (which < 3) next[e] = (long long)n_heads * 3 * d;
         to[e] = which * VLEN + (i / ROWS) * PAD + i % ROWS;
       } else if (idx - 5 * per_vec < n_v) {
         const int i = (idx - 5 * per_vec) * UNIT;
-        from[e] = (off_v + hd * dv + j0 + i) | (1 << 30);
+        from[e] = row + off_v + hd * dv + j0 + i;
         to[e] = 5 * VLEN + i;
       }
     }
-    auto fetch_group = [&](int p) {
+    auto fetch_group = [&](int p) {                   // the groups in their order
       for (int t = G * p; t < min(n, G * p + G); ++t) {
         float *dst = ring[t % DR_STAGES];
-        const float *row = proj + (size_t)(start + t) * ld;
-        const float *pr = prep + ((size_t)(start + t) * n_heads + hd) * 3 * d;
 #pragma unroll
         for (int e = 0; e < PER; ++e)
           if (to[e] >= 0) {
-            const float *src = (from[e] & (1 << 30)) ? row + (from[e] & ~(1 << 30)) : pr + from[e];
-            if (VEC) cp_async16_cg(dst + to[e], src);
-            else cp_async4(dst + to[e], src);
+            if (VEC) cp_async16_cg(dst + to[e], from[e]);
+            else cp_async4(dst + to[e], from[e]);
+            from[e] += next[e];
           }
       }
       cp_async_commit_group();
@@ -440,18 +480,23 @@ delta_rule_kernel(const float *proj, long long ld, int off_r, int off_k, int off
     return;
   }
 
-  // -------------------------------------------------------------- the two warps of the recurrence
+  // -------------------------------------------------------------- the warps of the recurrence
   const int sub = tid % LANES, col = tid / LANES;
   const int j = j0 + col;
-  const bool live = j < dv;
-  float S[ROWS];
+  const bool live = j < dv, stores = live && sub == 0;
+  f32x2 S[ROWS / 2];
   float *sp = state + (((size_t)seq_slot[b] * n_heads + hd) * dv + (live ? j : 0)) * d + sub * ROWS;
-#pragma unroll
-  for (int i = 0; i < ROWS; ++i) S[i] = (live && sub * ROWS + i < d) ? sp[i] : 0.f;
+  delta_load_state<ROWS>(S, sp, sub * ROWS, d, live);
+  float *o = out + (size_t)start * ldo + (size_t)hd * dv + j;       // the row that is stored next: the token before's
+  float acc = 0.f;
   auto token = [&](int t) {
     const float *slot = ring[t % DR_STAGES];
-    const float acc = delta_token<ROWS, LANES>(S, slot + sub * PAD, VLEN, slot[5 * VLEN + col]);
-    if (live && sub == 0) out[(size_t)(start + t) * ldo + (size_t)hd * dv + j] = acc;
+    float before = acc;
+    acc = delta_token<ROWS, LANES>(S, slot + sub * PAD, VLEN, slot[5 * VLEN + col], before);
+    if (t > 0) {
+      if (stores) *o = before;
+      o += ldo;
+    }
   };
   for (int p = 0; p < n_groups; ++p) {
     __syncthreads();
@@ -462,13 +507,12 @@ delta_rule_kernel(const float *proj, long long ld, int off_r, int off_k, int off
       for (int t = G * p; t < n; ++t) token(t);
     }
   }
+  acc = delta_sum<LANES>(acc);
+  if (stores && n > 0) *o = acc;
   // Only now may the next kernel's CTAs come onto the SMs: this kernel runs for as long as its longest sequence
   // with few warps to a CTA, and a dependent let in at the start would sit beside them in its wait for all that time.
   grid_dependents_launch();
-  if (live)
-#pragma unroll
-    for (int i = 0; i < ROWS; ++i)
-      if (sub * ROWS + i < d) sp[i] = S[i];
+  if (live) delta_store_state<ROWS>(S, sp, sub * ROWS, d);
 }
 
 static int launch_delta_scan(const float *proj, long long ld, int off_r, int off_k, int off_v, const float *prep, float *state,
@@ -563,10 +607,9 @@ delta_step_kernel(const float *proj, long long ld, int off_r, int off_k, int off
   const float *row = proj + (size_t)b * ld;
   const float *k = row + off_k + (size_t)hd * d;
   // this thread's share of its column of the state: on its way while the vectors are made
-  float S[ROWS];
+  f32x2 S[ROWS / 2];
   float *sp = state + (((size_t)seq_slot[b] * n_heads + hd) * d + (live ? col : 0)) * d + sub * ROWS;
-#pragma unroll
-  for (int i = 0; i < ROWS; ++i) S[i] = (live && sub * ROWS + i < d) ? sp[i] : 0.f;
+  delta_load_state<ROWS>(S, sp, sub * ROWS, d, live);
   for (int q = tid; q < rank; q += THREADS) th[q] = tanhf(row[off_x1 + q]);
   if (warp == 0) {                                    // the key's length: lane order, then the shuffle tree
     float ss = 0.f;
@@ -591,11 +634,10 @@ delta_step_kernel(const float *proj, long long ld, int off_r, int off_k, int off
     vals[i] = row[off_v + ch];
   }
   __syncthreads();
-  const float acc = delta_token<ROWS, LANES>(S, vecs + sub * PAD, VLEN, live ? vals[col] : 0.f);
+  float none = 0.f;
+  const float acc = delta_sum<LANES>(delta_token<ROWS, LANES>(S, vecs + sub * PAD, VLEN, live ? vals[col] : 0.f, none));
   if (live) {
-#pragma unroll
-    for (int i = 0; i < ROWS; ++i)
-      if (sub * ROWS + i < d) sp[i] = S[i];
+    delta_store_state<ROWS>(S, sp, sub * ROWS, d);
     if (sub == 0) outs[col] = acc;
   }
   __syncthreads();
