@@ -603,6 +603,48 @@ def test_32_bit_product_rows_do_not_depend_on_the_batch(K, N):
         assert torch.equal(out, rows[130][:M]), M
 
 
+# matrices that run on the tensor cores: rows of W and parts of K at the tiles' edges, eight parts (two to a CTA from 65 rows on), none
+@pytest.mark.parametrize("K,N", [(1024, 256), (1028, 257), (1060, 300), (2048, 2048), (2052, 9600), (8192, 384)])
+def test_32_bit_product_on_tensor_cores(K, N):
+    """A row has the same bits in every call.  Against 64 bits: each split leaves 2^-21 of a value at most and one product of two small parts
+    is left out (20 units of 2^-24 of |a| |w|), twelve sums of the tensor cores are cut and not rounded (24), K / 32 sums and those of the parts rounded."""
+    from libllm_b200.csrc import ops
+    a = rnd((300, K), "float32", 97)
+    w = rnd((N, K), "float32", 98)
+    bias = rnd((N,), "float32", 99)
+    full = torch.full((300, N), float("nan"), device=DEV)
+    ops.gemm_plain(a, w, full, bias)
+    ref = a.double() @ w.double().T + bias.double()
+    bound = (20 + 24 + K / 32 + 10) * 2 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double())
+    assert bool(((full.double() - ref).abs() <= bound).all())
+    for M in (1, 2, 16, 17, 32, 33, 64, 65, 128, 129):
+        out = torch.full((M, N), float("nan"), device=DEV)
+        ops.gemm_plain(a[:M], w, out, bias)
+        assert torch.equal(out, full[:M]), M
+
+
+def test_32_bit_product_on_tensor_cores_of_values_that_are_not_finite():
+    from libllm_b200.csrc import ops
+    K, N = 2048, 512
+    for M in (3, 40, 130):
+        a, w = rnd((M, K), "float32", 101), rnd((N, K), "float32", 102)
+        a[0, 5] = math.inf
+        a[1, 700] = -math.inf
+        a[2, 2047] = math.nan
+        w[7, 5] = 0.0                                  # infinity times nought
+        w[300, 9] = 3e38
+        a[M - 1, 9] = 2.0 if M > 3 else a[M - 1, 9]    # a product beyond the type's range
+        out = torch.empty((M, N), device=DEV)
+        ops.gemm_plain(a, w, out)
+        ref = a.double() @ w.double().T
+        want = torch.where(ref.abs() > 3.4028235e38, torch.copysign(torch.full_like(ref, math.inf), ref), ref)
+        assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+        assert torch.equal(out[torch.isinf(out)].double(), want[torch.isinf(want)])
+        ok = torch.isfinite(want)
+        bound = 130 * 2 ** -24 * (a.abs().double() @ w.abs().double().T)
+        assert bool(((out.double() - want).abs()[ok] <= bound[ok]).all())
+
+
 # widths of whole groups of 16 (gate and up rows in turns) and others; rows at the tiles' edges
 @pytest.mark.parametrize("M,I,K", [(1, 64, 64), (5, 173, 80), (8, 8192, 2048), (40, 300, 256), (200, 128, 136), (257, 391, 200),
                                    (1000, 1024, 512), (1, 16, 8), (16, 48, 136), (17, 80, 72), (33, 208, 200), (64, 1040, 64), (65, 48, 64),
