@@ -46,6 +46,7 @@ def lib() -> ctypes.CDLL:
             "llm_model_step": (c_int32, [PP, c_int32, I32P, I32P, I32P, I32P, I32P, I32P, c_char_p, F32P, F32P, I32P]),
             "llm_model_step_tokens": (c_int32, [PP, c_int32, I32P, I32P, I32P, I32P, I32P, c_char_p, F32P, PP]),
             "llm_pending_result": (c_int32, [PP, I32P]), "llm_pending_destroy": (c_int32, [PP]),
+            "llm_model_result_block": (c_int32, [PP, c_int64, PP, PP]), "llm_block_destroy": (c_int32, [PP]),
             "llm_model_synchronize": (c_int32, [PP]), "llm_model_stream": (c_int32, [PP, PP]),
             "llm_model_cache_info": (c_int32, [PP, PP]), "llm_model_cache_check": (c_int32, [PP]),
             "llm_model_debug_set_status": (c_int32, [PP, c_int32]), "llm_model_debug_wait_probe": (c_int32, [PP, c_int64]),

@@ -33,6 +33,13 @@ struct llm_completion_impl_t {
 struct llm_pending_impl_t {
   PendingTokens pending;
 };
+struct llm_block_impl_t {
+  std::shared_ptr<HostPool> pool;
+  void *data = nullptr;
+  ~llm_block_impl_t() {
+    if (pool) pool->give(data);
+  }
+};
 struct llm_cachebook_impl_t {
   std::unique_ptr<KVCache> cache;
 };
@@ -415,15 +422,35 @@ LLM_API int32_t llm_model_step(llm_model_t *m, int32_t n_items, const int32_t *s
     if (sampling_json) {
       const SamplingParams s = sampling_of(Json::parse(sampling_json, "sampling"));
       const StepResult r = e.step(items, &s, uniforms);
-      if (logits) e.read_logits(r, logits);
-      if (sampled) e.read_tokens(r, sampled);
-      if (!logits && !sampled) e.check_status();
+      e.read(r, logits, sampled);
     } else {
       const StepResult r = e.step(items);
-      if (logits) e.read_logits(r, logits);
-      else e.check_status();
+      e.read(r, logits, nullptr);
     }
   });
+}
+
+LLM_API int32_t llm_model_result_block(llm_model_t *m, int64_t bytes, llm_block_t *block, void **data) {
+  return guard_api([&] {
+    if (!block || !data) LLM_THROW(InvalidArg, "result_block: an output is null");
+    *block = nullptr;
+    *data = nullptr;
+    if (bytes <= 0) return;
+    const std::shared_ptr<HostPool> &pool = engine_of(m).host_pool();
+    std::unique_ptr<llm_block_impl_t> b(new llm_block_impl_t());
+    b->data = pool->take((size_t)bytes);
+    if (!b->data) return;
+    b->pool = pool;
+    *data = b->data;
+    *block = b.release();
+  });
+}
+LLM_API int32_t llm_block_destroy(llm_block_t *block) {
+  if (block && *block) {
+    delete *block;
+    *block = nullptr;
+  }
+  return STATUS_OK;
 }
 
 LLM_API int32_t llm_model_step_tokens(llm_model_t *m, int32_t n_items, const int32_t *slots, const int32_t *n_tokens,

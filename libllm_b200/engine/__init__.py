@@ -75,6 +75,20 @@ class PendingTokens:
             pass
 
 
+class _Block:
+    """A block of the model's page-locked host memory as an array's base: it goes back when no array looks at it any more."""
+
+    def __init__(self, block: c_void_p, address: int, shape: Tuple[int, ...]):
+        self._block = block
+        self.__array_interface__ = dict(version=3, typestr="<f4", shape=shape, data=(address, False))
+
+    def __del__(self):
+        try:
+            _lib.lib().llm_block_destroy(ctypes.byref(self._block))
+        except Exception:
+            pass
+
+
 def _int32(tokens: Sequence[int]) -> array:
     """Token ids as 32-bit integers.  A prompt's are converted by the array at once (2,048 of them: 324 -> 36 us); what it
     does not take (a float, a number beyond 32 bits) goes one by one, as ctypes takes it."""
@@ -247,6 +261,13 @@ class Engine:
         _lib.check(_lib.lib().llm_model_sequence_length(ctypes.byref(self._h), int(slot), ctypes.byref(n)))
         return n.value
 
+    def _rows(self, n: int) -> np.ndarray:
+        """Room for n rows of logits, in page-locked memory while there is some."""
+        shape = (n, self.vocab)
+        block, data = c_void_p(), c_void_p()
+        _lib.check(_lib.lib().llm_model_result_block(ctypes.byref(self._h), 4 * n * self.vocab, ctypes.byref(block), ctypes.byref(data)))
+        return np.asarray(_Block(block, data.value, shape)) if block else np.empty(shape, dtype=np.float32)
+
     def step(self, items: Sequence[StepItem], sampling: Optional[SamplingParams] = None,
              uniforms: Optional[Sequence[float]] = None, return_logits: bool = True):
         """Runs the items' tokens and returns the logits at the wanted places, float32
@@ -258,7 +279,7 @@ class Engine:
         W = len(want)
         if sampling is not None and uniforms is not None and len(uniforms) != W:
             raise InvalidArgError("one uniform number per wanted place is needed")
-        logits = np.empty((W, self.vocab), dtype=np.float32) if (return_logits or sampling is None) else None
+        logits = self._rows(W) if (return_logits or sampling is None) else None
         sampled = np.empty(max(W, 1), dtype=np.int32) if sampling is not None else None
         uni = None
         if sampling is not None and uniforms is not None:

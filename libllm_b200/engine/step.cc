@@ -141,7 +141,9 @@ Engine::Engine(std::unique_ptr<Model> model, const Options &options) : model_(st
     t.buf.allocate(sizeof(int) * ((size_t)last_capacity_ + 1));
     LLM_CUDA(cudaEventCreateWithFlags(&t.done, cudaEventDisableTiming));
   }
-  status_host_.allocate(sizeof(int));
+  status_host_.allocate(sizeof(int) * ((size_t)last_capacity_ + 1));
+  // three results of 64 rows of logits (a caller reads one while the next is computed), at most 96 MB
+  host_pool_.reset(new HostPool(std::min((size_t)96 << 20, 3 * 64 * sizeof(float) * (size_t)vocab())));
 }
 
 Engine::~Engine() {
@@ -315,17 +317,15 @@ StepResult Engine::step(const std::vector<StepItem> &items, const SamplingParams
   return out;
 }
 
-void Engine::read_logits(const StepResult &r, float *host) {
+void Engine::read(const StepResult &r, float *logits, int *tokens) {
   make_current();
-  if (r.n_rows > 0 && r.logits)
-    LLM_CUDA(cudaMemcpyAsync(host, r.logits, sizeof(float) * (size_t)r.n_rows * (size_t)vocab(), cudaMemcpyDeviceToHost, stream_));
+  if (logits && r.n_rows > 0 && r.logits)
+    LLM_CUDA(cudaMemcpyAsync(logits, r.logits, sizeof(float) * (size_t)r.n_rows * (size_t)vocab(), cudaMemcpyDeviceToHost, stream_));
+  const bool take = tokens && r.n_rows > 0 && r.tokens, staged = r.n_rows <= last_capacity_;
+  if (take)
+    LLM_CUDA(cudaMemcpyAsync(staged ? status_host_.as<int>() + 1 : tokens, r.tokens, sizeof(int) * (size_t)r.n_rows, cudaMemcpyDeviceToHost, stream_));
   check_status();
-}
-
-void Engine::read_tokens(const StepResult &r, int *host) {
-  make_current();
-  if (r.n_rows > 0 && r.tokens) LLM_CUDA(cudaMemcpyAsync(host, r.tokens, sizeof(int) * (size_t)r.n_rows, cudaMemcpyDeviceToHost, stream_));
-  check_status();
+  if (take && staged) memcpy(tokens, status_host_.as<int>() + 1, sizeof(int) * (size_t)r.n_rows);
 }
 
 // ---------------------------------------------------------------- eager path (prompts, mixed steps)

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "engine/model.h"
+#include "util/host_pool.h"
 
 namespace llm {
 
@@ -107,9 +108,10 @@ class Engine {
   // With it, a token is drawn at each wanted place; `uniforms` then holds one number in [0, 1) per
   // wanted place (null: zeros).  Returns when the work is queued on the engine's stream.
   StepResult step(const std::vector<StepItem> &items, const SamplingParams *sampling = nullptr, const float *uniforms = nullptr);
-  // Copies a step's logits to host memory, waits, and checks the status word.
-  void read_logits(const StepResult &r, float *host);
-  void read_tokens(const StepResult &r, int *host);
+  // Copies a step's logits and tokens (either may be null) to host memory, waits once, and checks the status word.
+  void read(const StepResult &r, float *logits, int *tokens);
+  // Where results for the host may lie so that the copy engine writes them directly.
+  const std::shared_ptr<HostPool> &host_pool() const { return host_pool_; }
 
   // Runs a step that samples one token per item (each wants exactly one place) and returns at
   // once: the tokens stay on the device (row i = item i), where the next step's items may take
@@ -174,7 +176,8 @@ class Engine {
   };
   std::vector<HostTokens> token_ring_;
   size_t token_turn_ = 0;
-  PinnedBuffer status_host_;
+  PinnedBuffer status_host_;         // the status word, then a step's tokens
+  std::shared_ptr<HostPool> host_pool_;
   std::map<GraphKey, std::unique_ptr<DecodeGraph>> graphs_[2];
   std::map<GraphKey, int> graph_turn_;
   DecodeGraph *last_graph_ = nullptr;

@@ -39,6 +39,7 @@ typedef struct llm_model_impl_t *llm_model_t;
 typedef struct llm_completion_impl_t *llm_completion_t;
 typedef struct llm_json_impl_t *llm_json_t;
 typedef struct llm_pending_impl_t *llm_pending_t;
+typedef struct llm_block_impl_t *llm_block_t;
 typedef struct llm_cachebook_impl_t *llm_cachebook_t;
 
 /* ---- global state */
@@ -98,6 +99,11 @@ int32_t llm_model_sequence_length(llm_model_t *m, int32_t slot, int32_t *length)
 int32_t llm_model_step(llm_model_t *m, int32_t n_items, const int32_t *slots, const int32_t *n_tokens, const int32_t *tokens,
                        const int32_t *fed_rows, const int32_t *n_want, const int32_t *want, const char *sampling_json,
                        const float *uniforms, float *logits, int32_t *sampled);
+/* A block of page-locked host memory that `logits` may point to: the copy then needs no staging and meets no page fault.  `block` and
+ * `data` are null where the model has none left; ordinary memory does as well.  The block stays valid until it is destroyed, also
+ * beyond the model's life, and may be destroyed by any thread. */
+int32_t llm_model_result_block(llm_model_t *m, int64_t bytes, llm_block_t *block, void **data);
+int32_t llm_block_destroy(llm_block_t *block);
 /* The same for steps that sample one token per item (each wants one place) without waiting: the
  * tokens stay on the device for the next step's fed_rows and arrive later in `pending`. */
 int32_t llm_model_step_tokens(llm_model_t *m, int32_t n_items, const int32_t *slots, const int32_t *n_tokens, const int32_t *tokens,

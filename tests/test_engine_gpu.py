@@ -247,3 +247,41 @@ def test_tensors_stored_in_other_types_load_to_the_same_model(dtype):
     s = engine.open_sequence()
     assert torch.equal(torch.from_numpy(engine.step([StepItem(s, toks, [0, 20, 39])])), outs[0])
     engine.close_sequence(s)
+
+
+def test_logits_stay_what_they_were_while_someone_holds_them():
+    """Results lie in a pool of the engine's: a block is lent again only when no array looks at it, with none left (more rows than it
+    holds) ordinary memory serves, and what is held outlives the engine."""
+    import gc
+
+    import numpy as np
+    from libllm_b200.engine import GREEDY, Engine, StepItem
+    engine = Engine.from_folder(model_folder("A"), dtype="float32", max_tokens=4096)
+    toks = tokens_for("A", 40, 3)
+
+    def rows(n, offset):
+        s = engine.open_sequence()
+        out = engine.step([StepItem(s, toks[offset:offset + n], list(range(n)))])
+        engine.close_sequence(s)
+        return out
+
+    first = rows(5, 0)
+    at, kept, part = first.ctypes.data, first.copy(), first[1:3]
+    for i in range(8):                                         # held: nobody else gets its place
+        other = rows(5, i + 1)
+        assert other.ctypes.data != at and np.array_equal(first, kept)
+    del first
+    gc.collect()
+    rows(5, 9)
+    assert np.array_equal(part, kept[1:3])                     # a slice of it holds it too
+    part = None
+    gc.collect()
+    again = rows(5, 0)
+    assert np.array_equal(again, kept) and again.flags.writeable
+    many = [rows(40, 0) for _ in range(8)]                     # 320 rows: more than the pool has
+    assert all(np.array_equal(m[:5], kept) for m in many)
+    s = engine.open_sequence()
+    logits, drawn = engine.step([StepItem(s, toks, [3, 39])], GREEDY, [0.0, 0.0])
+    assert np.array_equal(drawn, logits.argmax(-1)) and np.array_equal(logits, many[0][[3, 39]])
+    engine.close()
+    assert np.array_equal(again, kept) and all(np.array_equal(m, many[0]) for m in many)
