@@ -47,12 +47,22 @@ constexpr int TC_A_BYTES = TC_ROWS * TC_BK * 2;
 // lane holds both values of a feature (prompt steps); 3 like 1 with gate and up rows in turns of 16 (the map of get_gated_map: I a
 // multiple of 16), so that a warp has both halves of its features and trades them by shuffles: 64 tokens x 16,384
 // rows 19.7 -> 16.1 us, 8 tokens 14.4 -> 13.1.
-template <int TN, int SW>
+//
+// R, KBS (plain products): a matrix with few tiles of 128 rows leaves most SMs idle, and the others' time goes by the stages that a loader and an
+// issuer get through one by one, some 0.2 us each beyond the ring, whatever a stage holds (at K = 2,048 five ready stages of 32: 8.8 us for 6 tiles, 9.2
+// for 25).  There a tile has R = 32 or 64 rows and a stage KBS = 4 or 2 blocks of 64 of K, so that four or two times as many SMs each
+// get through a quarter or half of the stages.  The instruction keeps its 128 rows: those beyond R are whatever lies behind the
+// block in shared memory, and nobody reads their sums.  A row's sum is the same whatever R.  In steps of a few requests, K = 2,048: 3,104 rows
+// x 4 tokens 9.2 -> 7.2 us, 8,192 x 2 9.8 -> 7.5.  Every CTA brings the tokens too: from 33 tokens on 32 rows to a tile lose, and beyond 48 so do 64
+// (a prompt of 37 tokens, tiles of 128 / 64 / 32 rows: 1,054 / 1,043 / 1,070 us; a step of 64 50.0 / 50.6 ms a pass).
+template <int TN, int SW, int R = TC_ROWS, int KBS = 1>
 struct TcShape {
+  static_assert(SW == 0 || (R == TC_ROWS && KBS == 1), "gated units have tiles of 128 rows");
   static constexpr int A_TILES = SW == 2 ? 2 : 1;
-  static constexpr int A_BYTES = A_TILES * TC_A_BYTES;
+  static constexpr int A_BYTES = A_TILES * R * TC_BK * 2;
   static constexpr int B_BYTES = TN * TC_BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int BLOCK_BYTES = A_BYTES + B_BYTES;                  // 64 of K
+  static constexpr int STAGE_BYTES = KBS * BLOCK_BYTES;
   // Steps of few tokens (TN <= 32) take half of an SM's shared memory, so that the CTA of the next
   // product in the stream can move in beside this one and fill its ring with weights while this
   // one finishes; larger steps take a ring as deep as fits (measured: equal at 1 and 8 tokens,
@@ -62,7 +72,8 @@ struct TcShape {
   static constexpr int ACC_COLS = A_TILES * TN;                          // columns of one accumulator buffer
   static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;  // two buffers; a power of two
   static constexpr int XCH_BYTES = 64 * 17 * 4;                        // SwiGLU hand-over: 64 rows x 16 tokens (+1 pad)
-  static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + XCH_BYTES + 256;
+  static constexpr int BEYOND = (TC_ROWS - R) * TC_BK * 2;              // read behind the last block by the instruction's other rows
+  static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + BEYOND + XCH_BYTES + 256;
   static_assert(TMEM_COLS <= 512, "the accumulators do not fit tensor memory");
 };
 
@@ -92,17 +103,17 @@ __device__ __forceinline__ void store_turns(const float (&v)[16], TO *__restrict
   }
 }
 
-template <int TN, int SW, typename TO>
+template <int TN, int SW, typename TO, int R = TC_ROWS, int KBS = 1>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                TO *__restrict__ out, long long ldo, int M, int n_out, int K, int row_tiles, int tok_tiles,
                int k_parts, int kb_per_part, long long part_stride, int group_tiles, int group_rows, GluShape glu, int *status) {
-  using S = TcShape<TN, SW>;
+  using S = TcShape<TN, SW, R, KBS>;
   constexpr bool SWIGLU = SW == 1;                      // the interleaved tile with the hand-over
   constexpr int STAGES = S::STAGES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  unsigned char *xch_raw = smem + (size_t)STAGES * S::STAGE_BYTES;
+  unsigned char *xch_raw = smem + (size_t)STAGES * S::STAGE_BYTES + S::BEYOND;
   unsigned long long *bars = (unsigned long long *)(xch_raw + S::XCH_BYTES);
   // bars: full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], hand-over full and empty;
   // then the TMEM address and the abort flag
@@ -147,7 +158,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   const int n_tiles = row_tiles * tok_tiles * k_parts;
   const int n_kblocks_total = (K + TC_BK - 1) / TC_BK;
-  constexpr int ROWS_OUT = SW == 1 || SW == 3 ? 64 : 128;  // output features per tile
+  constexpr int ROWS_OUT = SW == 1 || SW == 3 ? 64 : R;  // output features per tile
 
   if (warp == 0) {
     // ------------------------------------------------------------ loader
@@ -169,11 +180,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       w.row_b = SW != 0 ? n_out + w.row_a : w.row_a + 64;
     };
     auto next = [&](Walk &w) {
-      if (++w.kb >= w.kb1) start(w, w.tile + gridDim.x);
+      w.kb += KBS;
+      if (w.kb >= w.kb1) start(w, w.tile + gridDim.x);
     };
     auto load_w = [&](const Walk &w, int stage) {
       const unsigned dst = smem_u32(smem + (size_t)stage * S::STAGE_BYTES);
-      if (leader) {
+      if (leader && (R < TC_ROWS || KBS > 1)) {
+        const int n = min(KBS, w.kb1 - w.kb);           // the part's last stage may have fewer blocks
+        mbar_expect_tx(bar_full + 8 * stage, n * S::BLOCK_BYTES);
+#pragma unroll
+        for (int j = 0; j < KBS; ++j)
+          if (j < n) tma_load_2d(dst + j * S::BLOCK_BYTES, &map_w, (w.kb + j) * TC_BK, w.row_a, bar_full + 8 * stage);
+      } else if (leader) {
         mbar_expect_tx(bar_full + 8 * stage, S::STAGE_BYTES);
         if (SW == 2) {                    // 128 gate rows, then 128 up rows: the map's boxes are 128 rows here
           tma_load_2d(dst, &map_w, w.kb * TC_BK, w.row_a, bar_full + 8 * stage);
@@ -188,8 +206,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     };
     auto load_x = [&](const Walk &w, int stage) {
       if (leader)
-        tma_load_2d(smem_u32(smem + (size_t)stage * S::STAGE_BYTES) + S::A_BYTES, &map_x, w.kb * TC_BK,
-                    w.x_row, bar_full + 8 * stage);
+#pragma unroll
+        for (int j = 0; j < KBS; ++j)
+          if (j == 0 || w.kb + j < w.kb1)
+            tma_load_2d(smem_u32(smem + (size_t)stage * S::STAGE_BYTES) + j * S::BLOCK_BYTES + S::A_BYTES, &map_x, (w.kb + j) * TC_BK,
+                        w.x_row, bar_full + 8 * stage);
     };
     // Weights first: they do not depend on the kernel before this one, so the whole ring
     // is filled with them while that kernel still runs.  Then the wait, then the tokens of
@@ -238,7 +259,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       if (!ok) break;
       tc_fence_after();
       const unsigned d_tmem = tmem_base + acc * S::ACC_COLS;
-      for (int kb = kb0; kb < kb1; ++kb) {
+      for (int kb = kb0; kb < kb1; kb += KBS) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, 3));
         if (!ok) break;
         tc_fence_after();
@@ -255,6 +276,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
               tc_mma(d_tmem + TN, a2_desc + (unsigned long long)(kk * 2), b_desc + (unsigned long long)(kk * 2), IDESC,
                      kk > 0 ? 1u : first);
           }
+#pragma unroll
+          for (int j = 1; j < KBS; ++j)
+            if (kb + j < kb1) {
+              const unsigned long long step = (unsigned long long)(j * (S::BLOCK_BYTES >> 4));
+#pragma unroll
+              for (int kk = 0; kk < TC_BK / 16; ++kk)
+                tc_mma(d_tmem, a_desc + step + (unsigned long long)(kk * 2), b_desc + step + (unsigned long long)(kk * 2), IDESC, 1u);
+            }
           tc_commit(bar_empty + 8 * stage);          // the stage is free when these products have read it
         }
         __syncwarp();
@@ -286,7 +315,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int row_in_tile = quarter * 32 + lane;
       const int tok0 = tok_tile * TN;
 #pragma unroll 1
-      for (int c0 = 0; c0 < TN && ok && (SW == 1 || tok0 + c0 < M); c0 += 16, ++n_chunk) {
+      for (int c0 = 0; c0 < TN && ok && (SW == 1 || tok0 + c0 < M) && quarter * 32 < R; c0 += 16, ++n_chunk) {
         float v[16];
         tc_ld16(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * S::ACC_COLS + c0), v);
         if (SW == 3) {
@@ -326,7 +355,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (lane == 0) mbar_arrive(bar_xempty);
           }
         } else {
-          const int f = row_tile * 128 + row_in_tile;
+          const int f = row_tile * R + row_in_tile;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const int tok = tok0 + c0 + i;
@@ -367,23 +396,23 @@ int get_gated_map(const void *W, long long I, long long K, CUtensorMap *out) {
   return LLM_OK;
 }
 
-template <int TN, int SW, typename TO>
+template <int TN, int SW, typename TO, int R = TC_ROWS, int KBS = 1>
 int launch_tc(const void *x, long long ldx, const void *W, void *out, long long ldo, int M, int N, int K, int k_parts,
               long long part_stride, const GluShape &glu, int *status, cudaStream_t stream, int n_groups = 1, int group_n = 0) {
-  using S = TcShape<TN, SW>;
+  using S = TcShape<TN, SW, R, KBS>;
   const int n_out = SW != 0 ? N / 2 : N;
-  const int rows_out = SW == 1 || SW == 3 ? 64 : 128;
+  const int rows_out = SW == 1 || SW == 3 ? 64 : R;
   const int row_tiles = (n_out + rows_out - 1) / rows_out;
   const int tok_tiles = (M + TN - 1) / TN;
   const int n_kblocks = (K + TC_BK - 1) / TC_BK;
   const int kb_per_part = (n_kblocks + k_parts - 1) / k_parts;
   LLM_REQUIRE((long long)(k_parts - 1) * kb_per_part < n_kblocks, "gemm_tc: %d parts leave one of them without work (K = %d)", k_parts, K);
   CUtensorMap map_w, map_x;
-  int rc = SW == 3 ? get_gated_map(W, n_out, K, &map_w) : get_map(W, N, K, K, SW == 2 ? 128 : 64, &map_w);
+  int rc = SW == 3 ? get_gated_map(W, n_out, K, &map_w) : get_map(W, N, K, K, SW == 2 ? 128 : R < 64 ? R : 64, &map_w);
   if (rc != LLM_OK) return rc;
   rc = get_map(x, (long long)n_groups * M, K, ldx, TN, &map_x);
   if (rc != LLM_OK) return rc;
-  auto kern = gemm_tc_kernel<TN, SW, TO>;
+  auto kern = gemm_tc_kernel<TN, SW, TO, R, KBS>;
   LLM_CHECK_CUDA(llm_allow_smem(kern, S::SMEM), "gemm_tc attribute");
   const long long tiles = (long long)row_tiles * tok_tiles * k_parts;
   LLM_REQUIRE(tiles < (1ll << 30), "gemm_tc: too many tiles");
@@ -641,6 +670,12 @@ bool takes_pair(int M, int N) {
   return N % 32 == 0 && M >= 512 && tok_tiles * GP_TOKENS * 4 <= (long long)M * 5 && tok_tiles * row_tiles * 2 >= sm_count();
 }
 
+// Rows of W to a tile of a plain product of few tokens: as many fewer than 128 as still leave every SM at most one tile (TcShape).
+int tile_rows(int N, int k_parts) {
+  const long long tiles = (long long)((N + TC_ROWS - 1) / TC_ROWS) * k_parts;
+  return tiles * 4 <= sm_count() ? 32 : tiles * 2 <= sm_count() ? 64 : TC_ROWS;
+}
+
 template <bool SWIGLU, typename TO>
 int dispatch_tc(const void *x, long long ldx, const void *W, void *out, long long ldo, int M, int N, int K, int k_parts,
                 long long part_stride, const GluShape &glu, int *status, cudaStream_t stream) {
@@ -657,6 +692,14 @@ int dispatch_tc(const void *x, long long ldx, const void *W, void *out, long lon
     if (takes_pair(M, N)) return launch_gated_pair<TO>(x, ldx, W, out, ldo, M, N / 2, K, glu, status, stream);
     TC_GO(128, 2);
   }
+#define TC_NARROW(TN, R, KBS) return launch_tc<TN, 0, TO, R, KBS>(x, ldx, W, out, ldo, M, N, K, k_parts, part_stride, glu, status, stream)
+  const int rows = M <= 48 ? tile_rows(N, k_parts) : TC_ROWS;
+  if (rows == 32 && M <= 16) TC_NARROW(16, 32, 4);
+  if (rows == 32 && M <= 32) TC_NARROW(32, 32, 4);
+  if (rows == 64 && M <= 16) TC_NARROW(16, 64, 2);
+  if (rows == 64 && M <= 32) TC_NARROW(32, 64, 2);
+  if (rows <= 64) TC_NARROW(64, 64, 2);
+#undef TC_NARROW
   if (M <= 16) TC_GO(16, 0);
   if (M <= 32) TC_GO(32, 0);
   if (M <= 64) TC_GO(64, 0);

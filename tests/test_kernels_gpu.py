@@ -661,6 +661,23 @@ def test_tensor_core_product_with_swiglu(M, I, K):
     close(out, P.swiglu(gu[:, :I], gu[:, I:]), "bfloat16")
 
 
+# tiles of 32 rows (up to 37 tiles of 128, parts counted; 32 tokens) and of 64 (up to 74, 48 tokens), the edges of a tile and of a stage of several blocks of K
+@pytest.mark.parametrize("M,N,K,parts", [(1, 4736, 8, 1), (16, 4737, 328, 1), (17, 31, 264, 1), (32, 9472, 128, 1), (33, 97, 1096, 1), (48, 4700, 520, 1), (49, 300, 136, 1),
+                                         (5, 2050, 1992, 2), (20, 1100, 2048, 5), (40, 1000, 1000, 4), (2, 9473, 192, 1)])
+def test_tensor_core_product_in_tiles_of_fewer_rows(M, N, K, parts):
+    """A row's sum is the same whatever the tile: the bits of the same rows in a matrix whose tiles have 128."""
+    from libllm_b200.csrc import ops
+    x = rnd((M, K), "bfloat16", 190)
+    w = rnd((N, K), "bfloat16", 191, std=0.1)
+    out = torch.full((parts, M, N), float("nan"), device=DEV) if parts > 1 else torch.full((M, N), float("nan"), device=DEV)
+    ops.gemm_tc(x, w, out)
+    wide = torch.cat([w, torch.zeros((19200 - N, K), dtype=torch.bfloat16, device=DEV)])       # 150 tiles of 128
+    ref = torch.full((parts, M, 19200), float("nan"), device=DEV) if parts > 1 else torch.full((M, 19200), float("nan"), device=DEV)
+    ops.gemm_tc(x, wide, ref)
+    ops.check_tc_status()
+    assert torch.equal(out, ref[..., :N])
+
+
 def test_tensor_core_product_rows_do_not_depend_on_the_batch():
     """A token's row is the same alone and among 200 others: each token is its own column of the tile."""
     from libllm_b200.csrc import ops
