@@ -57,7 +57,7 @@ constexpr int TC_A_BYTES = TC_ROWS * TC_BK * 2;
 // (a prompt of 37 tokens, tiles of 128 / 64 / 32 rows: 1,054 / 1,043 / 1,070 us; a step of 64 50.0 / 50.6 ms a pass).
 template <int TN, int SW, int R = TC_ROWS, int KBS = 1>
 struct TcShape {
-  static_assert(SW == 0 || (R == TC_ROWS && KBS == 1), "gated units have tiles of 128 rows");
+  static_assert(SW == 0 || (R == TC_ROWS && (KBS == 1 || SW == 3)), "gated units have tiles of 128 rows");
   static constexpr int A_TILES = SW == 2 ? 2 : 1;
   static constexpr int A_BYTES = A_TILES * R * TC_BK * 2;
   static constexpr int B_BYTES = TN * TC_BK * 2;
@@ -66,12 +66,16 @@ struct TcShape {
   // Steps of few tokens (TN <= 32) take half of an SM's shared memory, so that the CTA of the next
   // product in the stream can move in beside this one and fill its ring with weights while this
   // one finishes; larger steps take a ring as deep as fits (measured: equal at 1 and 8 tokens,
-  // 5 % faster at 64 with the deep ring).
-  static constexpr int BUDGET = TN <= 32 ? 100 * 1024 : 200 * 1024;
+  // 5 % faster at 64 with the deep ring).  The gated unit of up to 16 tokens, the widest product, takes stages of two blocks and as much as two CTAs
+  // of an SM can have: 8 tokens, 16 steps 14.35 -> 14.28 ms a pass (the other products too: 13.97, but decoders with more and smaller launches
+  // lose 1.5 %, whose kernels then find less room beside them; stages of two blocks in 73 KB: 15.5).
+  static constexpr int BUDGET = SW == 3 && TN == 16 ? 108 * 1024 : TN <= 32 ? 100 * 1024 : 200 * 1024;
   static constexpr int STAGES = BUDGET / STAGE_BYTES;
   static constexpr int ACC_COLS = A_TILES * TN;                          // columns of one accumulator buffer
   static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;  // two buffers; a power of two
-  static constexpr int XCH_BYTES = 64 * 17 * 4;                        // SwiGLU hand-over: 64 rows x 16 tokens (+1 pad)
+  // SwiGLU hand-over: 64 rows x 16 tokens (+1 pad).  Plain products have no use for it, but with 4 KB less of shared memory a third kernel's CTAs
+  // find room beside two of these, which costs a step of few tokens 1 to 2 % (8 tokens 14.28 -> 14.41 ms a pass).
+  static constexpr int XCH_BYTES = SW <= 1 ? 64 * 17 * 4 : 0;
   static constexpr int BEYOND = (TC_ROWS - R) * TC_BK * 2;              // read behind the last block by the instruction's other rows
   static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + BEYOND + XCH_BYTES + 256;
   static_assert(TMEM_COLS <= 512, "the accumulators do not fit tensor memory");
@@ -190,7 +194,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         mbar_expect_tx(bar_full + 8 * stage, n * S::BLOCK_BYTES);
 #pragma unroll
         for (int j = 0; j < KBS; ++j)
-          if (j < n) tma_load_2d(dst + j * S::BLOCK_BYTES, &map_w, (w.kb + j) * TC_BK, w.row_a, bar_full + 8 * stage);
+          if (j < n) {
+            if (SW == 3) tma_load_turns(dst + j * S::BLOCK_BYTES, &map_w, (w.kb + j) * TC_BK, w.row_a / 16, bar_full + 8 * stage);
+            else tma_load_2d(dst + j * S::BLOCK_BYTES, &map_w, (w.kb + j) * TC_BK, w.row_a, bar_full + 8 * stage);
+          }
       } else if (leader) {
         mbar_expect_tx(bar_full + 8 * stage, S::STAGE_BYTES);
         if (SW == 2) {                    // 128 gate rows, then 128 up rows: the map's boxes are 128 rows here
@@ -408,7 +415,7 @@ int launch_tc(const void *x, long long ldx, const void *W, void *out, long long 
   const int kb_per_part = (n_kblocks + k_parts - 1) / k_parts;
   LLM_REQUIRE((long long)(k_parts - 1) * kb_per_part < n_kblocks, "gemm_tc: %d parts leave one of them without work (K = %d)", k_parts, K);
   CUtensorMap map_w, map_x;
-  int rc = SW == 3 ? get_gated_map(W, n_out, K, &map_w) : get_map(W, N, K, K, SW == 2 ? 128 : R < 64 ? R : 64, &map_w);
+  int rc = SW == 3 ? get_gated_map(W, n_out, K, &map_w) : get_map(W, N, K, K, SW == 2 || KBS > 1 ? R : 64, &map_w);
   if (rc != LLM_OK) return rc;
   rc = get_map(x, (long long)n_groups * M, K, ldx, TN, &map_x);
   if (rc != LLM_OK) return rc;
@@ -682,7 +689,7 @@ int dispatch_tc(const void *x, long long ldx, const void *W, void *out, long lon
 #define TC_GO(TN, SW) return launch_tc<TN, SW, TO>(x, ldx, W, out, ldo, M, N, K, k_parts, part_stride, glu, status, stream)
   if (SWIGLU) {
     if (M <= 64 && N / 2 % 16 == 0) {
-      if (M <= 16) TC_GO(16, 3);
+      if (M <= 16) return launch_tc<16, 3, TO, TC_ROWS, 2>(x, ldx, W, out, ldo, M, N, K, k_parts, part_stride, glu, status, stream);
       if (M <= 32) TC_GO(32, 3);
       TC_GO(64, 3);
     }
