@@ -42,7 +42,7 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // (128 bytes of each row and part a stage, 16-byte asynchronous copies), so no barrier is met
 // before the parts are added.  A row's pitch of 36 floats spreads eight lanes' 16-byte reads over all banks.
 // W does not depend on the kernel before and is on its way before that has finished.
-// [2, 2,048] x [16,384, 2,048]^T: 285 -> 31 us (4.4 TB/s of W); [2, 8,192] x [2,048, 8,192]^T: 927 -> 20 us.
+// Measured at sizes that run on the tensor cores now: [2, 2,048] x [16,384, 2,048]^T 285 -> 31 us (4.4 TB/s of W); [2, 8,192] x [2,048, 8,192]^T 927 -> 20 us.
 template <int MT>
 struct FewShape {
   static constexpr int PITCH = PART_BLOCK + 4;
@@ -144,7 +144,7 @@ gemm_few_kernel(const float *A, long long lda, const float *__restrict__ W, long
 // whole tile over its own part of K from a ring of its own (no barriers), a lane 8 x 8 outputs: 16 reads of
 // 16 bytes for 128 packed multiplications and additions; and matrices of 2,048 rows, whose tiles alone would not
 // fill the SMs with warps, do.  Lanes take every fourth row of A and every eighth of W: with a pitch of 20 floats their reads meet no
-// bank twice.  [213, 2,048] x [16,384, 2,048]^T: 780 -> 416 us (34 TFLOP/s; tiles of 64 x 64 with single
+// bank twice.  [213, 2,048] x [16,384, 2,048]^T (on the tensor cores now): 780 -> 416 us (34 TFLOP/s; tiles of 64 x 64 with single
 // multiplications 463).
 struct TileShape {
   static constexpr int RM = 32, KS = 16, PITCH = KS + 4;
