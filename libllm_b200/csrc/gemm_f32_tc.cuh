@@ -10,7 +10,8 @@
 //   loader       TMA boxes of [128 x 32] of W and [TN x 32] of x (128-byte swizzle) into a ring; W's before the kernel before is waited for;
 //   converters   split W's tile and put both parts into tensor memory, as the A operand (a lane a row: shared memory, which the products and
 //                the copies keep busy, is read once for it), and split x's tile within shared memory;
-//   issuer       twelve tcgen05.mma a stage, into one of two accumulators (0.6 us at TN = 128, which bounds a stage there; splitting x 0.45 us);
+//   issuer       twelve tcgen05.mma a stage, into one of two accumulators (at TN = 128 a stage takes 0.9 us: 0.6 of products, 0.45 to split x, and three
+//                stages in the ring do not hide them and a load behind one another);
 //   adders       the sum of a stage (tcgen05.ld) to their registers.
 // K is cut into `parts` runs, one or two to each CTA of a cluster, whose sums meet through distributed shared memory and are added in order.
 // Two where TN is 128: such a CTA fills an SM, and sixteen clusters of eight do not find room at once.
