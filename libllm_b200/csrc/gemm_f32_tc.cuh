@@ -75,8 +75,11 @@ __device__ __forceinline__ float fs_peer(unsigned addr, unsigned rank) {        
 __device__ __forceinline__ void fs_put(unsigned addr, unsigned rank, float v) {
   asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, %1;\nst.shared::cluster.f32 [a], %2;\n}" ::"r"(addr), "r"(rank), "f"(v) : "memory");
 }
+__device__ __forceinline__ void fs_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fs_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fs_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  fs_cluster_arrive();
+  fs_cluster_wait();
 }
 
 template <int TN>
@@ -125,6 +128,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = *tmem_slot;
+  // A CTA's shared memory may be written by another one only when it is known to run: all say so here, and wait for it where the adders put their
+  // sums (the other warps where the parts meet), when it has long been so.
+  if (parts > 1) fs_cluster_arrive();
 
   const int tok0 = blockIdx.y * TN, row0 = blockIdx.z * 128;
   const int sub = parts > 1 ? SUB : 1;                          // parts of this CTA; the CTAs of a cluster share a tile's parts
@@ -299,6 +305,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           *y = parts == 1 && bias ? v + bias[row] : v;
         }
       }
+      if (parts > 1 && p == 0) {
+        __syncwarp();
+        fs_cluster_wait();
+      }
       if (parts > 1 && SUB == 1) {             // to the CTA that adds this row of x
         const int n_ctas = parts, most = (TN + n_ctas - 1) / n_ctas;
         const unsigned there = smem_u32(smem) + S::KEPT + (unsigned)((int)blockIdx.x * most * 128 + quarter * 32 + lane) * 4;
@@ -313,6 +323,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // ---------------------------------------------------------------- the parts' sums, in order
   if (parts > 1) {
     __syncwarp();
+    if (warp < S::ADD0) fs_cluster_wait();     // for the CTAs' start: the adders have
     fs_cluster_sync();
     const int n_ctas = parts / sub, rank = blockIdx.x;         // the grid's first dimension is one cluster
     const unsigned base = smem_u32(smem);

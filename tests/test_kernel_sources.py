@@ -112,3 +112,26 @@ def test_loads_from_tensor_memory_are_waited_for_where_they_are_issued():
                 assert depth >= 0, f"{file}: {name}: the block ends before the wait"
                 at += 1
     assert loads >= 10
+
+
+def calls(body, names):
+    """Where a body first calls one of these functions."""
+    return min((m.start() for m in re.finditer(r"\b(\w+)\s*(?:<[^;()]*>)?\(", body) if m.group(1) in names), default=None)
+
+
+def test_no_shared_memory_of_another_cta_is_touched_before_the_cluster_is_known_to_run():
+    """A CTA of a cluster may touch another one's shared memory only behind a cluster barrier that both have come to: until then that CTA need not be there."""
+    remote = {name for _, name, _, body, kernel in KERNELS if not kernel and "mapa" in body}
+    barrier = {name for _, name, _, body, kernel in KERNELS if not kernel and "barrier.cluster.wait" in body}
+    for _ in range(2):                                          # and what is made of them
+        barrier |= {name for _, name, _, body, kernel in KERNELS if not kernel and calls(body, barrier) is not None}
+        remote |= {name for _, name, _, body, kernel in KERNELS if not kernel and calls(body, remote) is not None}
+    seen, wrong = 0, []
+    for file, name, _, body, kernel in KERNELS:
+        first = calls(body, remote) if kernel else None
+        if first is not None:
+            seen += 1
+            known = calls(body, barrier)
+            if known is None or known > first:
+                wrong.append(f"{file}: {name}")
+    assert seen >= 4 and not wrong, (seen, wrong)
