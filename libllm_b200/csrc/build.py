@@ -46,7 +46,7 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fP
 # family -> (sources, headers it includes, extra flags, libraries)
 FAMILIES: Dict[str, dict] = {
     "elementwise": dict(sources=["elementwise.cu"], headers=["common.cuh"]),
-    "gemm_plain": dict(sources=["gemm_plain.cu"], headers=["common.cuh", "tc_common.cuh", "gemm_f32_tc.cuh"]),
+    "gemm_plain": dict(sources=["gemm_plain.cu"], headers=["common.cuh"]),
     "rope": dict(sources=["rope.cu"], headers=["common.cuh"]),
     "recurrent": dict(sources=["recurrent.cu"], headers=["common.cuh"]),
     "state_scan": dict(sources=["state_scan.cu"], headers=["common.cuh", "tc_common.cuh"]),

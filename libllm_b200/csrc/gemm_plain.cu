@@ -1,15 +1,15 @@
-// Plain matrix product C[M,N] = A[M,K] * W[N,K]^T (+ bias), 32-bit accumulate.  This is the matrix product of the true 32-bit path
-// (no reduced-precision mode) and the yardstick the fast bfloat16 products are tested
-// against.  The order in which an output's K products are added is fixed by the matrix alone, so a row's
+// Plain matrix product C[M,N] = A[M,K] * W[N,K]^T (+ bias) on the CUDA cores, 32-bit
+// accumulate.  This is the matrix product of the true 32-bit path (no tensor cores, no
+// reduced-precision mode) and the yardstick the fast bfloat16 products are tested
+// against.  The order in which an output's K products are added is fixed by K alone, so a row's
 // result does not depend on how many rows the call has or on where the row lies in the batch:
-// large 32-bit matrices run on the tensor cores, operands split so that nothing of 32-bit sums is lost (gemm_f32_tc.cuh); other 32-bit operands whose rows start on 16 bytes are added in eight parts of K (runs of whole
+// 32-bit operands whose rows start on 16 bytes are added in eight parts of K (runs of whole
 // blocks of 32), in each the even and the odd k by an accumulator each, ascending, and the parts in order;
 // everything else in the order k = 0, 1, 2, ... with one accumulator.
 //
 // Reference counterpart: the fp32 GEMM of the CPU backend (src/flint/cpu/matmul.cc:56-259)
 // and cublasGemmEx with CUBLAS_COMPUTE_32F on CUDA (src/flint/cuda/gemm_cublas.cc:160-197).
 #include "common.cuh"
-#include "gemm_f32_tc.cuh"
 
 LLM_DEFINE_LAST_ERROR(llm_gemm_plain_last_error)
 
@@ -42,7 +42,7 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // (128 bytes of each row and part a stage, 16-byte asynchronous copies), so no barrier is met
 // before the parts are added.  A row's pitch of 36 floats spreads eight lanes' 16-byte reads over all banks.
 // W does not depend on the kernel before and is on its way before that has finished.
-// Measured at sizes that run on the tensor cores now: [2, 2,048] x [16,384, 2,048]^T 285 -> 31 us (4.4 TB/s of W); [2, 8,192] x [2,048, 8,192]^T 927 -> 20 us.
+// [2, 2,048] x [16,384, 2,048]^T: 285 -> 31 us (4.4 TB/s of W); [2, 8,192] x [2,048, 8,192]^T: 927 -> 20 us.
 template <int MT>
 struct FewShape {
   static constexpr int PITCH = PART_BLOCK + 4;
@@ -144,7 +144,7 @@ gemm_few_kernel(const float *A, long long lda, const float *__restrict__ W, long
 // whole tile over its own part of K from a ring of its own (no barriers), a lane 8 x 8 outputs: 16 reads of
 // 16 bytes for 128 packed multiplications and additions; and matrices of 2,048 rows, whose tiles alone would not
 // fill the SMs with warps, do.  Lanes take every fourth row of A and every eighth of W: with a pitch of 20 floats their reads meet no
-// bank twice.  [213, 2,048] x [16,384, 2,048]^T (on the tensor cores now): 780 -> 416 us (34 TFLOP/s; tiles of 64 x 64 with single
+// bank twice.  [213, 2,048] x [16,384, 2,048]^T: 780 -> 416 us (34 TFLOP/s; tiles of 64 x 64 with single
 // multiplications 463).
 struct TileShape {
   static constexpr int RM = 32, KS = 16, PITCH = KS + 4;
@@ -268,25 +268,11 @@ static int launch_tile(const float *A, long long lda, const float *W, long long 
   }
   return LLM_OK;
 }
-// Whether a product runs on the tensor cores: a question of the matrix alone, never of the number of rows, so that a row has the same bits in
-// every call.  From K = 1,024 on its error against 64 bits is the smaller one (2-norm, normal operands: K = 1,028 1.5e-7 against the 1.7e-7 of the kernels
-// above, 2,048 1.5 to 2.0e-7 against 2.1e-7, 8,192 1.8e-7 against 4.1e-7; at 516 1.4e-7 against 1.35e-7, at 256 1.4e-7 against 1.0e-7).
-// Fewer than 256 rows of W are two tiles, which leave it no faster.  213 rows of x at [3,072, 2,048] / [2,048, 2,048] / [16,384, 2,048] / [2,048, 8,192]:
-// 97 / 66 / 409 / 230 -> 37 / 26 / 120 / 63 us; 64 at [16,384, 2,048] 130 -> 43; 2 rows, bound by the stream of W and what a
-// cluster costs: 10 / 8 / 37 / 21 -> 13 / 11 / 38 / 25 (alone).
-static bool takes_tc(int N, int K) { return N >= 256 && K >= 1024 && N <= 65535 * 128; }
 // Both kernels give a row the same bits, so the choice may look at everything.  Eight rows on the kernel for few cost 59 us at a W of
 // [16,384, 2,048] and 31 at [2,048, 8,192], the tile's kernel 76 and 119 whatever the rows up to 32: with tiles for
 // less than half of the SMs it is better to stream W twice.
 static int launch_f32(const float *A, long long lda, const float *W, long long ldw, const float *bias, float *C, long long ldc, int M, int N,
-                      int K, int *status, cudaStream_t stream) {
-  if (takes_tc(N, K)) {
-    if (M <= 16) return launch_f32_tc<16>(A, lda, W, ldw, bias, C, ldc, M, N, K, status, stream);
-    if (M <= 32) return launch_f32_tc<32>(A, lda, W, ldw, bias, C, ldc, M, N, K, status, stream);
-    if (M <= 64) return launch_f32_tc<64>(A, lda, W, ldw, bias, C, ldc, M, N, K, status, stream);
-    LLM_REQUIRE(M <= 65535 * BM, "gemm_plain: %d rows are too many", M);        // as for the tiles below
-    return launch_f32_tc<128>(A, lda, W, ldw, bias, C, ldc, M, N, K, status, stream);
-  }
+                      int K, cudaStream_t stream) {
   if (M == 1) return launch_few<1>(A, lda, W, ldw, bias, C, ldc, M, N, K, stream);
   if (M == 2) return launch_few<2>(A, lda, W, ldw, bias, C, ldc, M, N, K, stream);
   if (M <= 4) return launch_few<4>(A, lda, W, ldw, bias, C, ldc, M, N, K, stream);
@@ -368,13 +354,13 @@ static int launch(const void *A, long long lda, const void *W, long long ldw, co
 }
 
 // in_dtype is the type of A and W, out_dtype that of C.  Leading dimensions in elements.
-LLM_EXPORT int llm_gemm_plain_status(int in_dtype, int out_dtype, const void *A, long long lda, const void *W,
+LLM_EXPORT int llm_gemm_plain(int in_dtype, int out_dtype, const void *A, long long lda, const void *W,
                               long long ldw, const float *bias, void *C, long long ldc, int M, int N,
-                              int K, int *status, cudaStream_t stream) {
+                              int K, cudaStream_t stream) {
   if (M == 0) return LLM_OK;
   LLM_REQUIRE(M > 0 && N > 0 && K > 0 && lda >= K && ldw >= K && ldc >= N, "gemm_plain: bad sizes");
   if (in_dtype == LLM_F32 && out_dtype == LLM_F32 && takes_f32(A, lda, W, ldw, K))
-    return launch_f32((const float *)A, lda, (const float *)W, ldw, bias, (float *)C, ldc, M, N, K, status, stream);
+    return launch_f32((const float *)A, lda, (const float *)W, ldw, bias, (float *)C, ldc, M, N, K, stream);
   if (in_dtype == LLM_F32 && out_dtype == LLM_F32)
     return launch<float, float, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, stream);
   if (in_dtype == LLM_BF16 && out_dtype == LLM_BF16)
@@ -382,9 +368,4 @@ LLM_EXPORT int llm_gemm_plain_status(int in_dtype, int out_dtype, const void *A,
   if (in_dtype == LLM_BF16 && out_dtype == LLM_F32)
     return launch<__nv_bfloat16, __nv_bfloat16, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, stream);
   LLM_FAIL("gemm_plain: unsupported dtypes in %d out %d", in_dtype, out_dtype);
-}
-
-LLM_EXPORT int llm_gemm_plain(int in_dtype, int out_dtype, const void *A, long long lda, const void *W, long long ldw, const float *bias, void *C,
-                              long long ldc, int M, int N, int K, cudaStream_t stream) {
-  return llm_gemm_plain_status(in_dtype, out_dtype, A, lda, W, ldw, bias, C, ldc, M, N, K, nullptr, stream);
 }

@@ -288,16 +288,16 @@ void random_fill(void *out, DType dtype, long long n, unsigned long long seed, i
 }
 
 // ---------------------------------------------------------------- products
-LLM_KERNEL("gemm_plain", llm_gemm_plain_status, int, int, const void *, long long, const void *, long long, const float *, void *,
-           long long, int, int, int, int *, cudaStream_t)
+LLM_KERNEL("gemm_plain", llm_gemm_plain, int, int, const void *, long long, const void *, long long, const float *, void *,
+           long long, int, int, int, cudaStream_t)
 LLM_KERNEL("gemm_tc", llm_gemm_tc_glu, const void *, long long, const void *, void *, long long, int, int, int, int, int, float, float, float,
            int, long long, int *, cudaStream_t)
 LLM_KERNEL("gemv", llm_gemv_bf16, const void *, long long, const void *, void *, long long, int, int, int, int, int, int,
            long long, cudaStream_t)
 
-void gemm_plain(const Act &x, const Weight &w, const float *bias, const Act &out, int *status, cudaStream_t s) {
-  LLM_CALL("gemm_plain", llm_gemm_plain_status, code(x.dtype), code(out.dtype), x.data, (long long)x.ld, w.data(), (long long)w.cols,
-           bias, out.data, (long long)out.ld, (int)x.rows, (int)w.rows, (int)x.cols, status, s);
+void gemm_plain(const Act &x, const Weight &w, const float *bias, const Act &out, cudaStream_t s) {
+  LLM_CALL("gemm_plain", llm_gemm_plain, code(x.dtype), code(out.dtype), x.data, (long long)x.ld, w.data(), (long long)w.cols,
+           bias, out.data, (long long)out.ld, (int)x.rows, (int)w.rows, (int)x.cols, s);
 }
 bool gemm_tc_supported(const Act &x, const Weight &w) {
   return x.dtype == DType::BF16 && w.dtype == DType::BF16 && x.rows > 0 && x.cols % 8 == 0 && (x.rows == 1 || x.ld % 8 == 0) &&

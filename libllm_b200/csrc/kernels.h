@@ -77,7 +77,7 @@ void scale_rows(float *x, long long n, float scale, cudaStream_t s);
 void logit_transform(float *logits, long long n, float scale, float softcap, cudaStream_t s);
 void random_fill(void *out, DType dtype, long long n, unsigned long long seed, int law, float a, float b, cudaStream_t s);
 // ---- products
-void gemm_plain(const Act &x, const Weight &w, const float *bias, const Act &out, int *status, cudaStream_t s);
+void gemm_plain(const Act &x, const Weight &w, const float *bias, const Act &out, cudaStream_t s);
 bool gemm_tc_supported(const Act &x, const Weight &w);
 bool gemm_tc_pairs(const Act &x, const Weight &w);      // a gated unit of these sizes runs two SMs to a tile
 int gemm_tc_suggest_parts(int M, int N, int K);

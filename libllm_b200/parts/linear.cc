@@ -195,7 +195,7 @@ Act linear(StepContext &ctx, const Act &x, const Weight &w, const float *bias, D
     // the true 32-bit path; and, in bfloat16, a product with a bias (CUDA cores: such a model pays
     // for it, which load() says once)
     Act out = result_room(ctx, out_dtype, T, (int)w.rows, 1, parts_ok);
-    kernels::gemm_plain(x, w, bias, out, ctx.tc_status, ctx.stream);
+    kernels::gemm_plain(x, w, bias, out, ctx.stream);
     return out;
   }
   Act y = small_batch_linear(ctx, x, w, out_dtype, false, parts_ok);
@@ -224,7 +224,7 @@ Act linear(StepContext &ctx, const Act &x, const Weight &w, const float *bias, D
     log_warning("a bfloat16 product of width %lld runs on the CUDA cores: the tensor-core kernels want a width that is a "
                 "multiple of 8", (long long)x.cols);
   }
-  kernels::gemm_plain(x, w, nullptr, out, ctx.tc_status, ctx.stream);
+  kernels::gemm_plain(x, w, nullptr, out, ctx.stream);
   return out;
 }
 

@@ -603,27 +603,49 @@ def test_32_bit_product_rows_do_not_depend_on_the_batch(K, N):
         assert torch.equal(out, rows[130][:M]), M
 
 
-# matrices that run on the tensor cores: rows of W and parts of K at the tiles' edges, eight parts (two to a CTA from 65 rows on), none
+# widths and numbers of rows that whole models have, ragged ones beside them
 @pytest.mark.parametrize("K,N", [(1024, 256), (1028, 257), (1060, 300), (2048, 2048), (2052, 9600), (8192, 384)])
-def test_32_bit_product_on_tensor_cores(K, N):
-    """A row has the same bits in every call.  Against 64 bits: each split leaves 2^-21 of a value at most and one product of two small parts
-    is left out (20 units of 2^-24 of |a| |w|), twelve sums of the tensor cores are cut and not rounded (24), K / 32 sums and those of the parts rounded."""
+def test_32_bit_product_of_large_matrices(K, N):
+    """A row has the same bits in every call, from rows with gaps between them too, and the error against 64 bits is that of 32-bit additions."""
     from libllm_b200.csrc import ops
-    a = rnd((300, K), "float32", 97)
-    w = rnd((N, K), "float32", 98)
+    a = rnd((300, K + 8), "float32", 97)[:, :K]
+    w = rnd((N, K + 4), "float32", 98)[:, :K]
     bias = rnd((N,), "float32", 99)
-    full = torch.full((300, N), float("nan"), device=DEV)
-    ops.gemm_plain(a, w, full, bias)
+    full = torch.full((300, N + 3), float("nan"), device=DEV)
+    ops.gemm_plain(a, w, full[:, :N], bias)
+    assert bool(torch.isnan(full[:, N:]).all())
+    full = full[:, :N]
     ref = a.double() @ w.double().T + bias.double()
-    bound = (20 + 24 + K / 32 + 10) * 2 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double())
+    bound = (K / 8 + 40) * 2 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double())     # a part's chain of K / 8 and the parts'
     assert bool(((full.double() - ref).abs() <= bound).all())
-    for M in (1, 2, 16, 17, 32, 33, 64, 65, 128, 129):
+    whole, wide = a.contiguous(), w.contiguous()
+    for M in (1, 2, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129):
         out = torch.full((M, N), float("nan"), device=DEV)
-        ops.gemm_plain(a[:M], w, out, bias)
+        ops.gemm_plain(whole[:M], wide, out, bias)
         assert torch.equal(out, full[:M]), M
+    # operands of one sign: sums in 16 chains of K / 16 and 11 additions to join them, each addition off by 2^-23 / sqrt(12) of what it has so far at most (2-norm),
+    # a quarter above that for the share of small magnitudes
+    out = torch.empty((300, N), device=DEV)
+    ops.gemm_plain(whole.abs(), wide.abs(), out)
+    ref = whole.abs().double() @ wide.abs().double().T
+    assert float((out.double() - ref).norm() / ref.norm()) <= 1.25 * math.sqrt(K / 16 / 3 / 16 + 11 / 3) * 2 ** -23 / math.sqrt(12)
+    # a single product each is rounded once: nothing of the operands is left out
+    one = torch.zeros((64, K), device=DEV)
+    at = torch.arange(64, device=DEV) * (K // 64)
+    for value in (torch.ones(64, device=DEV), whole[:64, 0]):
+        one[torch.arange(64), at] = value
+        ops.gemm_plain(one, wide, out[:64])
+        assert torch.equal(out[:64], value[:, None] * wide[:, at].T)
+    # nor of values near the end of the type's range, down to where a product has fewer bits itself
+    for power in (-100, -126):
+        small = (whole[:64].double() * 2.0 ** power).float()
+        ops.gemm_plain(small, wide, out[:64])
+        ref = small.double() @ wide.double().T
+        bound = (K / 8 + 40) * 2 ** -24 * (small.abs().double() @ wide.abs().double().T) + K * 2.0 ** -149
+        assert bool(((out[:64].double() - ref).abs() <= bound).all()), power
 
 
-def test_32_bit_product_on_tensor_cores_of_values_that_are_not_finite():
+def test_32_bit_product_of_large_matrices_with_values_that_are_not_finite():
     from libllm_b200.csrc import ops
     K, N = 2048, 512
     for M in (3, 40, 130):
@@ -641,7 +663,7 @@ def test_32_bit_product_on_tensor_cores_of_values_that_are_not_finite():
         assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
         assert torch.equal(out[torch.isinf(out)].double(), want[torch.isinf(want)])
         ok = torch.isfinite(want)
-        bound = 130 * 2 ** -24 * (a.abs().double() @ w.abs().double().T)
+        bound = (K / 8 + 40) * 2 ** -24 * (a.abs().double() @ w.abs().double().T)
         assert bool(((out.double() - want).abs()[ok] <= bound[ok]).all())
 
 
