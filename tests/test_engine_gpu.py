@@ -255,7 +255,7 @@ def test_logits_stay_what_they_were_while_someone_holds_them():
     import gc
 
     import numpy as np
-    from libllm_b200.engine import GREEDY, Engine, StepItem
+    from libllm_b200.engine import GREEDY, Engine, StepItem, _Block
     engine = Engine.from_folder(model_folder("A"), dtype="float32", max_tokens=4096)
     toks = tokens_for("A", 40, 3)
 
@@ -278,8 +278,16 @@ def test_logits_stay_what_they_were_while_someone_holds_them():
     gc.collect()
     again = rows(5, 0)
     assert np.array_equal(again, kept) and again.flags.writeable
-    many = [rows(40, 0) for _ in range(8)]                     # 320 rows: more than the pool has
+    # a model of 256 words has a pool of 2 MB: 51 results of 40 rows.  Beyond them ordinary memory serves
+    lent = lambda array: isinstance(array.base, _Block)  # noqa: E731
+    many = [rows(40, 0) for _ in range(60)]
+    places = [lent(m) for m in many]
+    assert lent(again) and 40 <= sum(places) <= 51 and places == sorted(places, reverse=True)
     assert all(np.array_equal(m[:5], kept) for m in many)
+    at, many[7] = many[7].ctypes.data, None                    # a place in the middle comes back and is lent again
+    gc.collect()
+    many[7] = rows(40, 0)
+    assert lent(many[7]) and many[7].ctypes.data == at and not lent(rows(40, 0))
     s = engine.open_sequence()
     logits, drawn = engine.step([StepItem(s, toks, [3, 39])], GREEDY, [0.0, 0.0])
     assert np.array_equal(drawn, logits.argmax(-1)) and np.array_equal(logits, many[0][[3, 39]])
