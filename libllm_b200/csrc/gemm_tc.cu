@@ -66,15 +66,17 @@ struct TcShape {
   // Steps of few tokens (TN <= 32) take half of an SM's shared memory, so that the CTA of the next
   // product in the stream can move in beside this one and fill its ring with weights while this
   // one finishes; larger steps take a ring as deep as fits (measured: equal at 1 and 8 tokens,
-  // 5 % faster at 64 with the deep ring).  The gated unit of up to 16 tokens, the widest product, takes stages of two blocks and as much as two CTAs
-  // of an SM can have: 8 tokens, 16 steps 14.35 -> 14.28 ms a pass (the other products too: 13.97, but decoders with more and smaller launches
+  // 5 % faster at 64 with the deep ring).  Tiles of fewer rows take BEYOND besides: with 32 rows, and with 64 rows and up to 16 tokens, that makes 116,224
+  // bytes, of which two lack 1 KB of an SM; such a CTA has room beside tiles of 128 rows or the gated unit, not beside one of its kind.  The
+  // gated unit of up to 16 tokens, the widest product, takes stages of two blocks and as much as two CTAs
+  // of an SM can have: 8 tokens, 16 steps 14.35 -> 14.23 ms a pass (the other products too: 13.97, but decoders with more and smaller launches
   // lose 1.5 %, whose kernels then find less room beside them; stages of two blocks in 73 KB: 15.5).
   static constexpr int BUDGET = SW == 3 && TN == 16 ? 108 * 1024 : TN <= 32 ? 100 * 1024 : 200 * 1024;
   static constexpr int STAGES = BUDGET / STAGE_BYTES;
   static constexpr int ACC_COLS = A_TILES * TN;                          // columns of one accumulator buffer
   static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;  // two buffers; a power of two
   // SwiGLU hand-over: 64 rows x 16 tokens (+1 pad).  Plain products have no use for it, but with 4 KB less of shared memory a third kernel's CTAs
-  // find room beside two of these, which costs a step of few tokens 1 to 2 % (8 tokens 14.28 -> 14.41 ms a pass).
+  // find room beside two of these, which costs a step of few tokens 1 to 2 % (tiles of 128 rows, 8 tokens: 14.28 -> 14.41 ms a pass; not tried with tiles of fewer).
   static constexpr int XCH_BYTES = SW <= 1 ? 64 * 17 * 4 : 0;
   static constexpr int BEYOND = (TC_ROWS - R) * TC_BK * 2;              // read behind the last block by the instruction's other rows
   static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + BEYOND + XCH_BYTES + 256;

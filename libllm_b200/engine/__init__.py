@@ -273,7 +273,10 @@ class Engine:
         """Runs the items' tokens and returns the logits at the wanted places, float32
         [wanted, vocab] in the order of the items and of their ``want``.  With ``sampling`` it
         returns (logits or None, tokens): a token drawn at each wanted place; ``uniforms`` then
-        holds one number in [0, 1) per wanted place."""
+        holds one number in [0, 1) per wanted place.
+
+        The logits may lie in page-locked memory that the engine lends for as long as an array looks at any of them, and such an
+        array cannot be resized in place: copy the rows that are to be kept for long."""
         items = list(items)
         slots, n_tok, toks, fed, n_want, want = _flatten(items)
         W = len(want)
